@@ -639,7 +639,7 @@ def run_ours(args):
 
     bound_name, _ = _rl.bound(flops_pos, bytes_pos, fp32_peak or 77.0, hbm_peak)
     kernel_name = {1: "position_kernel<128,128,1024,1>", 2: "gd128_kernel"}.get(
-        args.schedule, "position_grouped_kernel<1024>")
+        args.schedule, "wave_gd_kernel<128>")
     if bound_name == "hbm":
         roof = {"bound": "hbm", "achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": hbm_achieved / hbm_peak, "peak_source": hbm_source + ", of measured"}

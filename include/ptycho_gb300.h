@@ -507,12 +507,13 @@ int ptycho_gd_batch_noalloc(const ptycho_geometry* geometry, void* object, void*
  * Kernel schedule for the fused per-position kernel of a given ROI edge length:
  * 0 = library default, 1 = shared-memory Stockham passes (every ROI and
  * variant), 2 = register-resident four-step transform (128 x 128 single-slice
- * gradient descent only; other cases fall back to 1), 3 = shared-memory passes
- * by groups of warps that each own 16 rows / columns, with block-wide barriers
- * only between the axes of a transform (128 x 128: gradient descent of every
- * model, projection sets of one slice and probe, the position correction of
- * single-slice batches; other cases fall back to 1). The default is 3 where it
- * applies, else 1. Process-wide; results agree between schedules to float32
+ * gradient descent only; other cases fall back to 1), 3 = packed
+ * shared-memory passes by warps that each own 8 rows / columns, with block-wide
+ * barriers only between the axes of a transform (128 x 128: every model and
+ * option but projection sets with kept far fields and the position correction
+ * of multislice batches, on arrays aligned to 16 bytes; other cases fall back
+ * to 1). The default is 3 where it applies, else 1; other square ROIs have only
+ * the default. Process-wide; results agree between schedules to float32
  * rounding. Returns the previous setting (0-3), or -PTYCHO_ERR_INVALID_ARGUMENT
  * for a schedule outside 0-3 (the setting is then unchanged).
  * No reference counterpart (tuning knob of this library's autotuner).

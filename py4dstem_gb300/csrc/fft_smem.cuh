@@ -260,10 +260,19 @@ __device__ __forceinline__ float2 cis_rounded(float phi) {
   }
   const DF x{phi, 0.0f};
   const DF x2 = df_mul(x, x);
-  DF s{kCoefs.shi[11], kCoefs.slo[11]};
-  DF c{kCoefs.chi[11], kCoefs.clo[11]};
+  // the terms from n = 7 on are below 2^-30 (sine) and 2^-26 (cosine): single
+  // floats carry them without moving a rounded result
+  constexpr int kSingle = 7;
+  float sf = kCoefs.shi[11], cf = kCoefs.chi[11];
 #pragma unroll
-  for (int n = 10; n >= 0; --n) {
+  for (int n = 10; n >= kSingle; --n) {
+    sf = fmaf(sf, x2.hi, kCoefs.shi[n]);
+    cf = fmaf(cf, x2.hi, kCoefs.chi[n]);
+  }
+  DF s{sf, 0.0f};
+  DF c{cf, 0.0f};
+#pragma unroll
+  for (int n = kSingle - 1; n >= 0; --n) {
     s = df_add(df_mul(s, x2), DF{kCoefs.shi[n], kCoefs.slo[n]});
     c = df_add(df_mul(c, x2), DF{kCoefs.chi[n], kCoefs.clo[n]});
   }

@@ -4,6 +4,7 @@
 // on the caller's stream.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -151,6 +152,11 @@ Workspace workspace_layout(int Sx, int Sy, int Px, int Py, int T, int M, int B,
   w.com = take(sizeof(double) * 4);
   w.red = take(sizeof(double) * 1024);
   w.total = off;
+  // (square regions only: the wave kernels read it)
+  const size_t pitch = ((size_t)Py + Sy + 3) / 2;
+  w.total_trans = Sx == Sy && !staged
+                      ? std::max(off, align256(w.obj_grad + 2 * sizeof(float4) * T * Px * pitch))
+                      : off;
   return w;
 }
 
@@ -168,6 +174,7 @@ void bind_workspace(BatchArgs& a, void* base, const Workspace& w) {
   a.err = reinterpret_cast<float*>(p + w.err);
   a.err_part = reinterpret_cast<float*>(p + w.err_part);
   a.det_f = reinterpret_cast<float2*>(p + w.det_f);
+  a.trans = reinterpret_cast<float4*>(p + w.obj_grad);
   a.obj_grad = reinterpret_cast<float2*>(p + w.obj_grad);
   a.obj_nrm = reinterpret_cast<float*>(p + w.obj_nrm);
   a.tile_max = reinterpret_cast<float*>(p + w.tile_max);
@@ -210,6 +217,7 @@ int prepare(const ptycho_geometry* g, int32_t batch, void* workspace, size_t wor
   a.potential = g->object_is_potential;
   a.B = batch;
   bind_workspace(a, workspace, w);
+  if (workspace_bytes < w.total_trans) a.trans = nullptr;
   return PTYCHO_OK;
 }
 
@@ -251,7 +259,7 @@ size_t ptycho_workspace_bytes(const ptycho_geometry* g, int32_t max_batch) {
   return workspace_layout(g->roi_x, g->roi_y, g->object_x, g->object_y, g->num_slices,
                           g->num_probes, max_batch, (g->flags & PTYCHO_FLAG_KEEP_FARFIELD) != 0,
                           detector_x(g), detector_y(g))
-      .total;
+      .total_trans;
 }
 
 static int run_batch(const ptycho_geometry* g, void* object, void* probe,
@@ -286,6 +294,7 @@ static int run_batch(const ptycho_geometry* g, void* object, void* probe,
                                  a.M == 1 && !a.mixed_formula
                              ? 1
                              : 0;
+  a.probe_rows = a.staging_t ? 0 : position_probe_rows(a);
   e = a.staging_t ? launch_position_v2(a, s) : launch_position_kernel(a, s);
   if (e != cudaSuccess) return cuda_fail(e, "position kernel");
   e = launch_reduce_and_update(a, s);
@@ -443,6 +452,7 @@ int ptycho_gd_gradient(const ptycho_geometry* g, const void* object, const void*
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = launch_probe_spectrum(a, s);
   if (e != cudaSuccess) return cuda_fail(e, "probe spectrum kernel");
+  a.probe_rows = position_probe_rows(a);
   e = launch_position_kernel(a, s);  // natural staging order (the shared-memory schedule)
   if (e != cudaSuccess) return cuda_fail(e, "position kernel");
   e = launch_gradient(a, object_grad, static_cast<float2*>(probe_grad), loss, s);

@@ -30,6 +30,7 @@ struct BatchArgs {
   int exact_probe_grad;    // probe term through the adjoint of the sub-pixel shift
   int prepare_spectrum;    // after the probe update, the next batch's probe spectrum
   int nobj_only;           // object reduction of the |P|^2 terms alone (probe overlap)
+  int probe_rows;          // rows of st_probe that hold probe terms (0: one per position)
   int nprobe_from_object;  // plain single-slice GD: the probe side gathers |O|^2 from the
                            // object instead of reading staged terms (none are written)
   const float* aperture;   // (N) Fourier amplitude of the initial probe (aperture constraint)
@@ -66,6 +67,9 @@ struct BatchArgs {
   float* err;           // (B)
   float* err_part;      // (B, chunks) per-chunk error partials of the staged path
   float2* det_f;        // (B,M,Ax Ay) detector-grid far fields (resampling only)
+  float4* trans;        // two shifted copies of the transmission functions
+                        // (ptycho_wave.cuh), or null without room for them; shares
+                        // the memory of the reduction outputs below
   float2* obj_grad;     // (T,P)
   float* obj_nrm;       // (T,P)
   float* tile_max;      // (T,ntiles)
@@ -82,6 +86,9 @@ struct Workspace {
   size_t probe_spec, tw, st_obj, st_nobj, st_probe, st_nprobe, scratch_f, st_pm, pos_round, err,
       err_part, det_f, obj_grad, obj_nrm, tile_max, probe_part, probe_npart, probe_bmax,
       probe_grad, probe_nrm, com, red, total;
+  // total with the transmission copies, which start at obj_grad; a workspace of
+  // at least `total` but less than this runs the general position kernels
+  size_t total_trans;
 };
 
 // Ax, Ay: detector shape (resampling when it differs from Sx, Sy)
@@ -109,6 +116,8 @@ void timing_after(cudaStream_t s);
 // Launchers (return cudaError_t of the last launch).
 cudaError_t launch_probe_spectrum(const BatchArgs& a, cudaStream_t s);
 cudaError_t launch_position_kernel(const BatchArgs& a, cudaStream_t s);
+// BatchArgs::probe_rows of the position kernel this batch will run.
+int position_probe_rows(const BatchArgs& a);
 cudaError_t launch_position_correction(const BatchArgs& a, cudaStream_t s);
 cudaError_t launch_probe_inverse(const BatchArgs& a, cudaStream_t s);
 // |P_b|^2 of the shifted probe (mode 0) of every batch position into st_nobj.

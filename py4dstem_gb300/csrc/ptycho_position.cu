@@ -10,6 +10,7 @@ namespace pty {
 
 #define PTY_DECLARE_SIZE(S)                                                         \
   cudaError_t launch_position_kernel_##S(const BatchArgs& a, cudaStream_t s);       \
+  int position_probe_rows_##S(const BatchArgs& a);                                  \
   cudaError_t launch_position_correction_##S(const BatchArgs& a, cudaStream_t s);   \
   cudaError_t launch_probe_inverse_##S(const BatchArgs& a, cudaStream_t s);         \
   cudaError_t launch_probe_intensity_##S(const BatchArgs& a, cudaStream_t s);        \
@@ -40,6 +41,18 @@ bool roi_supported(int Sx, int Sy) {
       return true;
     default:
       return false;
+  }
+}
+
+int position_probe_rows(const BatchArgs& a) {
+  if (staged_batch(a)) return 0;
+  switch (roi_key(a.Sx, a.Sy)) {
+    case roi_key(32, 32): return position_probe_rows_32(a);
+    case roi_key(48, 48): return position_probe_rows_48(a);
+    case roi_key(64, 64): return position_probe_rows_64(a);
+    case roi_key(96, 96): return position_probe_rows_96(a);
+    case roi_key(128, 128): return position_probe_rows_128(a);
+    default: return 0;
   }
 }
 

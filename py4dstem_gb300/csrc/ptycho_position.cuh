@@ -16,10 +16,9 @@
 //                   multislice back-transmits and back-propagates chi
 //                                  (ptychographic_methods.py:1818-1908, 2353-2565, 2906-3093)
 // The adjoint terms go to position-major staging buffers; ptycho_reduce.cu sums
-// them over positions in a fixed order. position_one runs every phase with the
-// whole block; position_grouped_128 (the default at 128 x 128) runs the same
-// model with 8 groups of warps that synchronise among themselves between the
-// turns of its transforms.
+// them over positions in a fixed order. These are the general kernels: any
+// supported region, every option. Square regions run the packed kernels of
+// ptycho_wave.cuh instead wherever those apply (use_wave below).
 //
 // This header holds the kernel templates; ptycho_position_<S>.cu instantiates
 // them for one region-of-interest edge S each (the translation units compile in
@@ -666,605 +665,6 @@ __global__ void __launch_bounds__(NT, 1) position_kernel(BatchArgs a) {
   position_one<SX, SY, NT, kMode>(a, blockIdx.x, red);
 }
 
-// The per-position model at 128 x 128 (kKind, see position_grouped_kernel) with
-// the block split into 8 groups of 4 warps. A group owns 16 rows in the
-// real-space phases and 16 columns in the Fourier-space phases; its elementwise
-// work and its share of each 2D transform (the same Stockham passes and
-// twiddles as fft2d, on its own lines) synchronise through a named barrier of
-// its 128 threads. A block-wide barrier is needed only where a transform turns
-// from one axis to the other (one per transform: 4 per position of single-slice
-// gradient descent instead of the 24 of the block-wide schedule), and between
-// them the groups drift apart in phase (one
-// loading from memory while another runs its passes). To need no extra turn,
-// the inverse transforms run columns then rows and the forward ones rows then
-// columns (fft2d: rows then columns both ways), so results agree with the
-// block-wide schedule to rounding, not bit for bit.
-//   real space (row group g):      x = 16 g + i,          y = t        (i < 16)
-//   Fourier space (column group g): x = t / 16 + 8 i,     y = 16 g + t % 16
-// for thread t < 128 of the group; both walks are bank-conflict free on the
-// pitch-129 wave and coalesced in global memory.
-template <int NT, int kKind>
-__device__ __forceinline__ void position_grouped_128(const BatchArgs& a, const int b,
-                                                     float* red) {
-  constexpr int S = 128;
-  using L = Layout<S, S>;
-  constexpr int N = L::N;
-  constexpr int LD = L::LD;
-  constexpr int GT = 128;                // threads per group
-  constexpr int G = NT / GT;             // groups
-  constexpr int LINES = S / G;           // rows (columns) a group owns
-  constexpr int PER = LINES * S / GT;    // samples per thread
-  constexpr int CH = 8;                  // global loads in flight per thread
-  static_assert(NT == 1024 && LINES == 16 && PER == 16, "grouped 128 x 128 layout");
-  extern __shared__ float4 smem4[];
-  float2* buf = reinterpret_cast<float2*>(smem4);
-  float2* twx = buf + S * LD;
-  float2* twy = twx + S;
-  float2* rpx = twy + S;
-  float2* rpy = rpx + S;
-
-  const int tid = threadIdx.x;
-  const int g = tid / GT;
-  const int tg = tid % GT;
-  const GroupSync gsync{1 + g, GT};
-  const int prow = a.pos_rows ? a.pos_rows[b] : b;
-  const int arow = a.amp_rows ? a.amp_rows[b] : b;
-  const bool pos_ok = isfinite(a.positions[2 * prow]) && isfinite(a.positions[2 * prow + 1]);
-  const float posx = finite_or_zero(a.positions[2 * prow]);
-  const float posy = finite_or_zero(a.positions[2 * prow + 1]);
-  const float rx = rintf(posx);  // numpy.round: half to even
-  const float ry = rintf(posy);
-  const float dx = posx - rx;
-  const float dy = posy - ry;
-  const int x0 = (int)rx;
-  const int y0 = (int)ry;
-  const float invN = 1.0f / (float)N;
-  const float* amp = a.amplitudes + (size_t)arow * N;
-
-  for (int i = tid; i < S; i += NT) {
-    twx[i] = a.tw[i];
-    twy[i] = a.tw[S + i];
-    const float k = (float)fint(i, S) / (float)S;
-    rpx[i] = cis_rounded(__fmul_rn(__fmul_rn(-6.2831855f, k), dx));
-  }
-  for (int i = tid - S; i >= 0 && i < S; i += NT) {
-    const float k = (float)fint(i, S) / (float)S;
-    rpy[i] = cis_rounded(__fmul_rn(__fmul_rn(-6.2831855f, k), dy));
-  }
-  if (tid == 0) a.pos_round[b] = make_int2(x0, y0);
-  __syncthreads();
-
-  const int bx = pmod(x0 - S / 2, a.Px);
-  const int by = pmod(y0 - S / 2, a.Py);
-  auto obj_x = [&](int x) {
-    const int t = bx + (x + S / 2) % S;
-    return t >= a.Px ? t - a.Px : t;
-  };
-  auto obj_y = [&](int y) {
-    const int t = by + (y + S / 2) % S;
-    return t >= a.Py ? t - a.Py : t;
-  };
-  // sample i of this thread in either walk
-  const int ry0 = LINES * g;                // real space: rows ry0 + i, column tg
-  const int fx0 = tg / LINES;               // Fourier space: rows fx0 + 8 i,
-  const int fy = LINES * g + tg % LINES;    //   column fy
-  constexpr int FXS = GT / LINES;
-  float2* const rows_g = buf + ry0 * LD;    // the group's rows
-  float2* const cols_g = buf + LINES * g;   // the group's columns
-
-  // the transforms of the group's lines: forward = rows then columns (real
-  // space in, Fourier space out), inverse = columns then rows
-  auto forward = [&]() {
-    Schedule<S>::template run<LINES, GT, -1>(rows_g, LD, 1, twy, tg, gsync);
-    __syncthreads();
-    Schedule<S>::template run<LINES, GT, -1>(cols_g, 1, LD, twx, tg, gsync);
-  };
-  auto inverse = [&]() {
-    Schedule<S>::template run<LINES, GT, +1>(cols_g, 1, LD, twx, tg, gsync);
-    __syncthreads();
-    Schedule<S>::template run<LINES, GT, +1>(rows_g, LD, 1, twy, tg, gsync);
-  };
-  // shifted probe of mode m: spectrum x ramps, inverse transform (columns,
-  // then rows)
-  auto shifted_probe = [&](int m) {
-    const float2* __restrict__ spec = a.probe_spec + (size_t)m * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float2 sv[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) sv[i] = __ldg(spec + (fx0 + FXS * (c0 + i)) * S + fy);
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = fx0 + FXS * (c0 + i);
-        buf[x * LD + fy] = c_mul(sv[i], c_mul(rpx[x], rpy[fy]));
-      }
-    }
-    gsync();
-    inverse();
-  };
-  shifted_probe(0);
-
-  // A exp(i angle F) - F on the group's columns, one division per pixel;
-  // returns this thread's share of sum (A - |F|)^2. keep (or null) receives F
-  // unmasked, for the position correction after the batch update.
-  auto project = [&](float2* keep) {
-    float err = 0.0f;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float av[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) av[i] = __ldg(amp + (fx0 + FXS * (c0 + i)) * S + fy);
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = fx0 + FXS * (c0 + i);
-        const int e = x * S + fy;
-        const int idx = x * LD + fy;
-        float2 f = buf[idx];
-        if (keep) keep[e] = f;
-        const float mk = a.det_mask ? a.det_mask[e] : 1.0f;
-        if (a.det_mask) f = c_scale(f, mk);
-        const float af = c_abs(f);
-        const float A = av[i];
-        const float d = A - af;
-        err += d * d;
-        const float q = af > 0.0f ? A / af : 0.0f;
-        float2 r = af > 0.0f ? make_float2(fmaf(f.x, q, -f.x), fmaf(f.y, q, -f.y))
-                             : c_sub(make_float2(A, 0.0f), f);
-        if (a.det_mask) r = c_scale(r, mk);
-        buf[idx] = r;
-      }
-    }
-    return err;
-  };
-  float err = 0.0f;
-
-  if constexpr (kKind == 0 || kKind == 5) {
-    // psi = P O; P stashed for the adjoint
-    float2* pst = a.st_probe + (size_t)b * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float2 ov[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) ov[i] = load_object(a, 0, obj_x(ry0 + c0 + i), obj_y(tg));
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = ry0 + c0 + i;
-        const float2 p = c_scale(buf[x * LD + tg], invN);
-        pst[x * S + tg] = p;
-        buf[x * LD + tg] = c_mul(p, ov[i]);
-      }
-    }
-    gsync();
-    forward();
-    err = project(kKind == 5 ? a.scratch_f + (size_t)b * N : nullptr);
-    gsync();
-    inverse();
-
-    // adjoint terms: conj(P) chi (or the potential's), |P|^2, conj(O) chi
-    float2* gobj = a.st_obj + (size_t)b * N;
-    float* nobj = a.st_nobj + (size_t)b * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float2 ov[CH], pv[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = ry0 + c0 + i;
-        ov[i] = load_object(a, 0, obj_x(x), obj_y(tg));
-        pv[i] = pst[x * S + tg];
-      }
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = ry0 + c0 + i;
-        const int e = x * S + tg;
-        const float2 chi = c_scale(buf[x * LD + tg], invN);
-        gobj[e] = object_term(a.potential, ov[i], pv[i], chi);
-        nobj[e] = c_abs2(pv[i]);
-        pst[e] = c_conj_mul(ov[i], chi);
-        // (plain gradient descent leaves |O|^2 to the probe side's gather from
-        // the object; with kept far fields the probe side reads it staged)
-        if constexpr (kKind == 5) a.st_nprobe[(size_t)b * N + e] = c_abs2(ov[i]);
-      }
-    }
-  } else if constexpr (kKind == 1) {
-    // multislice: P_{s+1} = IFFT2(FFT2(O_s P_s) H_s), each P_s stashed in its
-    // slice's object-term row (the adjoint overwrites it with the term)
-    const int T = a.T;
-    // buf (Fourier space, the group's columns) times H or conj(H)
-    auto propagate = [&](const float2* __restrict__ h, bool conjugate) {
-#pragma unroll 1
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 hv[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) hv[i] = __ldg(h + (fx0 + FXS * (c0 + i)) * S + fy);
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int idx = (fx0 + FXS * (c0 + i)) * LD + fy;
-          buf[idx] = c_mul(buf[idx], conjugate ? make_float2(hv[i].x, -hv[i].y) : hv[i]);
-        }
-      }
-    };
-    for (int s = 0; s < T; ++s) {
-      float2* pst = a.st_obj + ((size_t)s * a.B + b) * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 ov[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) ov[i] = load_object(a, s, obj_x(ry0 + c0 + i), obj_y(tg));
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int x = ry0 + c0 + i;
-          const float2 p = c_scale(buf[x * LD + tg], invN);
-          pst[x * S + tg] = p;
-          buf[x * LD + tg] = c_mul(ov[i], p);
-        }
-      }
-      gsync();
-      if (s + 1 < T) {
-        forward();
-        propagate(a.props + (size_t)s * N, false);
-        gsync();
-        inverse();
-      }
-    }
-    forward();  // far field of the last slice's exit wave
-    err = project(nullptr);
-    gsync();
-    inverse();
-    // adjoint, slice by slice backwards; chi conj(O_s) goes back through the
-    // propagator into the slice before, at slice 0 it is the probe term
-    for (int s = T - 1; s >= 0; --s) {
-      float2* pst = a.st_obj + ((size_t)s * a.B + b) * N;
-      float* nst = a.st_nobj + ((size_t)s * a.B + b) * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 ov[CH], pv[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int x = ry0 + c0 + i;
-          ov[i] = load_object(a, s, obj_x(x), obj_y(tg));
-          pv[i] = pst[x * S + tg];
-        }
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int x = ry0 + c0 + i;
-          const int e = x * S + tg;
-          const int idx = x * LD + tg;
-          const float2 chi = c_scale(buf[idx], invN);
-          pst[e] = object_term(a.potential, ov[i], pv[i], chi);
-          nst[e] = c_abs2(pv[i]);
-          const float2 bt = c_mul(chi, make_float2(ov[i].x, -ov[i].y));  // chi conj(O_s)
-          if (s > 0) {
-            buf[idx] = bt;
-          } else {
-            a.st_probe[(size_t)b * N + e] = bt;
-            a.st_nprobe[(size_t)b * N + e] = c_abs2(ov[i]);
-          }
-        }
-      }
-      if (s > 0) {
-        gsync();
-        forward();
-        propagate(a.props + (size_t)(s - 1) * N, true);
-        gsync();
-        inverse();
-      }
-    }
-  } else if constexpr (kKind == 4) {
-    // mixed-state multislice gradient descent: every mode through every slice,
-    // P_{s+1,m} = IFFT2(FFT2(O_s P_{s,m}) H_s) with each P_{s,m} stashed; the far
-    // fields F_m share the ratio A / sqrt(sum_m |F_m|^2); each mode's adjoint
-    // walks back through the slices, summing its terms into slice s's rows
-    const int T = a.T, M = a.M;
-    float* itot = reinterpret_cast<float*>(rpy + S);  // N, indexed by Fourier pixel
-    auto propagate = [&](const float2* __restrict__ h, bool conjugate) {
-#pragma unroll 1
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 hv[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) hv[i] = __ldg(h + (fx0 + FXS * (c0 + i)) * S + fy);
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int idx = (fx0 + FXS * (c0 + i)) * LD + fy;
-          buf[idx] = c_mul(buf[idx], conjugate ? make_float2(hv[i].x, -hv[i].y) : hv[i]);
-        }
-      }
-    };
-    for (int m = 0; m < M; ++m) {
-      if (m > 0) shifted_probe(m);
-      for (int s = 0; s < T; ++s) {
-        float2* pst = a.st_pm + (((size_t)s * a.B + b) * M + m) * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-        for (int c0 = 0; c0 < PER; c0 += CH) {
-          float2 ov[CH];
-#pragma unroll
-          for (int i = 0; i < CH; ++i)
-            ov[i] = load_object(a, s, obj_x(ry0 + c0 + i), obj_y(tg));
-#pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            const int x = ry0 + c0 + i;
-            const float2 p = c_scale(buf[x * LD + tg], invN);
-            pst[x * S + tg] = p;
-            buf[x * LD + tg] = c_mul(ov[i], p);
-          }
-        }
-        gsync();
-        if (s + 1 < T) {
-          forward();
-          propagate(a.props + (size_t)s * N, false);
-          gsync();
-          inverse();
-        }
-      }
-      forward();
-      float2* f = a.scratch_f + ((size_t)b * M + m) * N;
-      for (int i = 0; i < PER; ++i) {
-        const int x = fx0 + FXS * i;
-        const int e = x * S + fy;
-        const float2 v = buf[x * LD + fy];
-        f[e] = v;
-        const float av = hypotf(v.x, v.y);  // |F_m|^2 as numpy forms it
-        itot[e] = (m == 0 ? 0.0f : itot[e]) + av * av;
-      }
-    }
-    for (int i = 0; i < PER; ++i) {
-      const int e = (fx0 + FXS * i) * S + fy;
-      const float mk = a.det_mask ? a.det_mask[e] : 1.0f;
-      float tot = sqrtf(itot[e]);
-      if (a.det_mask) tot = sqrtf(itot[e] * mk * mk);
-      const float A = __ldg(amp + e);
-      const float d = A - tot;
-      err += d * d;
-      itot[e] = tot == 0.0f ? 0.0f : A / tot;
-    }
-    for (int m = 0; m < M; ++m) {
-      // (the previous mode's adjoint read the wave by rows)
-      if (m > 0) __syncthreads();
-      const float2* f = a.scratch_f + ((size_t)b * M + m) * N;
-      for (int i = 0; i < PER; ++i) {
-        const int x = fx0 + FXS * i;
-        const int e = x * S + fy;
-        const float mk = a.det_mask ? a.det_mask[e] : 1.0f;
-        float2 fv = f[e];
-        if (a.det_mask) fv = c_scale(fv, mk);
-        float2 r = c_sub(c_scale(fv, itot[e]), fv);
-        if (a.det_mask) r = c_scale(r, mk);
-        buf[x * LD + fy] = r;
-      }
-      gsync();
-      inverse();
-      for (int s = T - 1; s >= 0; --s) {
-        const float2* pst = a.st_pm + (((size_t)s * a.B + b) * M + m) * N;
-        float2* gobj = a.st_obj + ((size_t)s * a.B + b) * N;
-        float* nobj = a.st_nobj + ((size_t)s * a.B + b) * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-        for (int c0 = 0; c0 < PER; c0 += CH) {
-          float2 ov[CH], pv[CH];
-#pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            const int x = ry0 + c0 + i;
-            ov[i] = load_object(a, s, obj_x(x), obj_y(tg));
-            pv[i] = pst[x * S + tg];
-          }
-#pragma unroll
-          for (int i = 0; i < CH; ++i) {
-            const int x = ry0 + c0 + i;
-            const int e = x * S + tg;
-            const int idx = x * LD + tg;
-            const float2 chi = c_scale(buf[idx], invN);
-            const float2 g = object_term(a.potential, ov[i], pv[i], chi);
-            const float pn = c_abs2(pv[i]);
-            if (m == 0) {
-              gobj[e] = g;
-              nobj[e] = pn;
-            } else {
-              gobj[e] = c_add(gobj[e], g);
-              nobj[e] = nobj[e] + pn;
-            }
-            const float2 bt = c_mul(chi, make_float2(ov[i].x, -ov[i].y));  // chi conj(O_s)
-            if (s > 0) {
-              buf[idx] = bt;
-            } else {
-              a.st_probe[((size_t)b * M + m) * N + e] = bt;
-              if (m == 0) a.st_nprobe[(size_t)b * N + e] = c_abs2(ov[i]);
-            }
-          }
-        }
-        if (s > 0) {
-          gsync();
-          forward();
-          propagate(a.props + (size_t)(s - 1) * N, true);
-          gsync();
-          inverse();
-        }
-      }
-    }
-  } else if constexpr (kKind == 3) {
-    // projection sets, single slice and probe: the factor c psi + (1 - c) w of
-    // the exit wave w is projected, A exp(i angle F); the new exit wave
-    // x w + a psi + b projected is kept and is chi of the adjoint
-    const float px_ = 1.0f - a.pa - a.pb;
-    const float py_ = 1.0f - a.pc;
-    float2* pst = a.st_probe + (size_t)b * N;
-    float2* ew = a.exit_waves + (size_t)prow * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float2 ov[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) ov[i] = load_object(a, 0, obj_x(ry0 + c0 + i), obj_y(tg));
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = ry0 + c0 + i;
-        const int e = x * S + tg;
-        const float2 p = c_scale(buf[x * LD + tg], invN);
-        pst[e] = p;
-        const float2 psi = c_mul(p, ov[i]);
-        const float2 w = a.ew_valid ? ew[e] : psi;
-        buf[x * LD + tg] = c_add(c_scale(psi, a.pc), c_scale(w, py_));
-      }
-    }
-    gsync();
-    forward();
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float av[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) av[i] = __ldg(amp + (fx0 + FXS * (c0 + i)) * S + fy);
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = fx0 + FXS * (c0 + i);
-        const int e = x * S + fy;
-        const int idx = x * LD + fy;
-        float2 f = buf[idx];
-        if (a.det_mask) f = c_scale(f, a.det_mask[e]);
-        const float af = c_abs(f);
-        const float A = av[i];
-        const float d = A - af;
-        err += d * d;
-        const float q = af > 0.0f ? A / af : 0.0f;
-        buf[idx] = af > 0.0f ? c_scale(f, q) : make_float2(A, 0.0f);
-      }
-    }
-    gsync();
-    inverse();
-    float2* gobj = a.st_obj + (size_t)b * N;
-    float* nobj = a.st_nobj + (size_t)b * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float2 ov[CH], pv[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = ry0 + c0 + i;
-        ov[i] = load_object(a, 0, obj_x(x), obj_y(tg));
-        pv[i] = pst[x * S + tg];
-      }
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int x = ry0 + c0 + i;
-        const int e = x * S + tg;
-        const float2 proj = c_scale(buf[x * LD + tg], invN);
-        const float2 psi = c_mul(pv[i], ov[i]);
-        const float2 w = a.ew_valid ? ew[e] : psi;
-        const float2 chi =
-            c_add(c_add(c_scale(w, px_), c_scale(psi, a.pa)), c_scale(proj, a.pb));
-        ew[e] = chi;
-        gobj[e] = object_term(a.potential, ov[i], pv[i], chi);
-        nobj[e] = c_abs2(pv[i]);
-        pst[e] = c_conj_mul(ov[i], chi);
-        a.st_nprobe[(size_t)b * N + e] = c_abs2(ov[i]);
-      }
-    }
-  } else {
-    // mixed state: the far fields F_m of every mode share the ratio
-    // A / sqrt(sum_m |F_m|^2) (0 where the model is 0); F_m wait in scratch_f
-    const int M = a.M;
-    float* itot = reinterpret_cast<float*>(rpy + S);  // N, indexed by Fourier pixel
-    for (int m = 0; m < M; ++m) {
-      if (m > 0) shifted_probe(m);
-      float2* pst = a.st_probe + ((size_t)b * M + m) * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 ov[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) ov[i] = load_object(a, 0, obj_x(ry0 + c0 + i), obj_y(tg));
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int x = ry0 + c0 + i;
-          const float2 p = c_scale(buf[x * LD + tg], invN);
-          pst[x * S + tg] = p;
-          buf[x * LD + tg] = c_mul(p, ov[i]);
-        }
-      }
-      gsync();
-      forward();
-      float2* f = a.scratch_f + ((size_t)b * M + m) * N;
-      for (int i = 0; i < PER; ++i) {
-        const int x = fx0 + FXS * i;
-        const int e = x * S + fy;
-        const float2 v = buf[x * LD + fy];
-        f[e] = v;
-        const float av = hypotf(v.x, v.y);  // |F_m|^2 as numpy forms it
-        itot[e] = (m == 0 ? 0.0f : itot[e]) + av * av;
-      }
-    }
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-    for (int c0 = 0; c0 < PER; c0 += CH) {
-      float av[CH];
-#pragma unroll
-      for (int i = 0; i < CH; ++i) av[i] = __ldg(amp + (fx0 + FXS * (c0 + i)) * S + fy);
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        const int e = (fx0 + FXS * (c0 + i)) * S + fy;
-        const float mk = a.det_mask ? a.det_mask[e] : 1.0f;
-        float tot = sqrtf(itot[e]);
-        if (a.det_mask) tot = sqrtf(itot[e] * mk * mk);
-        const float A = av[i];
-        const float d = A - tot;
-        err += d * d;
-        itot[e] = tot == 0.0f ? 0.0f : A / tot;
-      }
-    }
-    float2* gobj = a.st_obj + (size_t)b * N;
-    float* nobj = a.st_nobj + (size_t)b * N;
-    for (int m = 0; m < M; ++m) {
-      // (the previous mode's adjoint read the wave by rows)
-      if (m > 0) __syncthreads();
-      const float2* f = a.scratch_f + ((size_t)b * M + m) * N;
-      for (int i = 0; i < PER; ++i) {
-        const int x = fx0 + FXS * i;
-        const int e = x * S + fy;
-        const float mk = a.det_mask ? a.det_mask[e] : 1.0f;
-        float2 fv = f[e];
-        if (a.det_mask) fv = c_scale(fv, mk);
-        float2 r = c_sub(c_scale(fv, itot[e]), fv);
-        if (a.det_mask) r = c_scale(r, mk);
-        buf[x * LD + fy] = r;
-      }
-      gsync();
-      inverse();
-      float2* pst = a.st_probe + ((size_t)b * M + m) * N;
-#pragma unroll 1  // (unrolled, the chunks' live values spill)
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 ov[CH], pv[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int x = ry0 + c0 + i;
-          ov[i] = load_object(a, 0, obj_x(x), obj_y(tg));
-          pv[i] = pst[x * S + tg];
-        }
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int x = ry0 + c0 + i;
-          const int e = x * S + tg;
-          const float2 chi = c_scale(buf[x * LD + tg], invN);
-          const float2 g = object_term(a.potential, ov[i], pv[i], chi);
-          const float pn = c_abs2(pv[i]);
-          if (m == 0) {
-            gobj[e] = g;
-            nobj[e] = pn;
-            a.st_nprobe[(size_t)b * N + e] = c_abs2(ov[i]);
-          } else {
-            gobj[e] = c_add(gobj[e], g);
-            nobj[e] = nobj[e] + pn;
-          }
-          pst[e] = c_conj_mul(ov[i], chi);
-        }
-      }
-    }
-  }
-  const float tot = block_sum<NT>(err, red);
-  if (tid == 0) a.err[b] = pos_ok ? tot : __int_as_float(0x7fc00000);
-}
-
-// kKind: gradient descent 0 single slice, 1 multislice, 2 mixed state (single
-// slice), 4 mixed-state multislice, 5 single slice keeping the far fields for
-// the position correction; 3 projection sets (single slice and probe)
-template <int NT, int kKind>
-__global__ void __launch_bounds__(NT, 1) position_grouped_kernel(BatchArgs a) {
-  __shared__ float red[NT / 32];
-  position_grouped_128<NT, kKind>(a, blockIdx.x, red);
-}
-
-
 // Position correction of one batch (ptychographic_methods.py:2071-2225), run
 // after the batch's object update. One block per position:
 //   F0_m = FFT2(P_m O_old)        kept by the forward pass in scratch_f
@@ -1478,191 +878,27 @@ __global__ void __launch_bounds__(NT, 1) position_correction_kernel(BatchArgs a)
   if (tid == 0) correction_update(a, prow, posx, posy, pos_ok, s5);
 }
 
-// Position correction of a single-slice batch at 128 x 128 with the passes and
-// walks of position_grouped_kernel: per mode and direction the shifted probe
-// (Fourier space by columns, inverse transform), times the moved object patch
-// (real space by rows), forward transform, and the gradient term against the
-// kept far field (Fourier space by columns); the normal-equation sums walk the
-// same columns. Same expressions as position_correction_kernel.
-template <int NT>
-__global__ void __launch_bounds__(NT, 1) position_correction_grouped_kernel(BatchArgs a) {
-  constexpr int S = 128;
-  using L = Layout<S, S>;
-  constexpr int N = L::N;
-  constexpr int LD = L::LD;
-  constexpr int GT = 128;
-  constexpr int G = NT / GT;
-  constexpr int LINES = S / G;
-  constexpr int PER = LINES * S / GT;
-  constexpr int CH = 8;
-  constexpr int FXS = GT / LINES;
-  static_assert(NT == 1024 && LINES == 16 && PER == 16, "grouped 128 x 128 layout");
-  extern __shared__ float4 smem4[];
-  float2* buf = reinterpret_cast<float2*>(smem4);
-  float2* twx = buf + S * LD;
-  float2* twy = twx + S;
-  float2* rpx = twy + S;
-  float2* rpy = rpx + S;
-  __shared__ double red[5][NT / 32];
+}  // namespace
+}  // namespace pty
 
-  const int b = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int g = tid / GT;
-  const int tg = tid % GT;
-  const GroupSync gsync{1 + g, GT};
-  const int M = a.M;
-  const int prow = a.pos_rows ? a.pos_rows[b] : b;
-  const int arow = a.amp_rows ? a.amp_rows[b] : b;
-  const bool pos_ok = isfinite(a.positions_rw[2 * prow]) && isfinite(a.positions_rw[2 * prow + 1]);
-  const float posx = finite_or_zero(a.positions_rw[2 * prow]);
-  const float posy = finite_or_zero(a.positions_rw[2 * prow + 1]);
-  const float rx = rintf(posx);
-  const float ry = rintf(posy);
-  const float dx = posx - rx;
-  const float dy = posy - ry;
-  const int x0 = (int)rx;
-  const int y0 = (int)ry;
-  const float invN = 1.0f / (float)N;
+#include "ptycho_wave.cuh"
 
-  for (int i = tid; i < S; i += NT) {
-    twx[i] = a.tw[i];
-    twy[i] = a.tw[S + i];
-    const float k = (float)fint(i, S) / (float)S;
-    rpx[i] = cis_rounded(__fmul_rn(__fmul_rn(-6.2831855f, k), dx));
-  }
-  for (int i = tid - S; i >= 0 && i < S; i += NT) {
-    const float k = (float)fint(i, S) / (float)S;
-    rpy[i] = cis_rounded(__fmul_rn(__fmul_rn(-6.2831855f, k), dy));
-  }
-  __syncthreads();
+namespace pty {
+namespace {
 
-  const int bx = pmod(x0 - S / 2, a.Px);
-  const int by = pmod(y0 - S / 2, a.Py);
-  const int ry0 = LINES * g;
-  const int fx0 = tg / LINES;
-  const int fy = LINES * g + tg % LINES;
-  float2* const rows_g = buf + ry0 * LD;
-  float2* const cols_g = buf + LINES * g;
-  auto forward = [&]() {
-    Schedule<S>::template run<LINES, GT, -1>(rows_g, LD, 1, twy, tg, gsync);
-    __syncthreads();
-    Schedule<S>::template run<LINES, GT, -1>(cols_g, 1, LD, twx, tg, gsync);
-  };
-  auto inverse = [&]() {
-    Schedule<S>::template run<LINES, GT, +1>(cols_g, 1, LD, twx, tg, gsync);
-    __syncthreads();
-    Schedule<S>::template run<LINES, GT, +1>(rows_g, LD, 1, twy, tg, gsync);
-  };
-  // object column of this thread's real-space samples, and the object row of
-  // sample i, with the patch moved one pixel along x (dir 0) or y (dir 1)
-  auto obj_col = [&](int dir) {
-    int t2 = by + (tg + S / 2) % S;
-    if (t2 >= a.Py) t2 -= a.Py;
-    if (dir == 1) t2 = t2 + 1 == a.Py ? 0 : t2 + 1;
-    return t2;
-  };
-  auto obj_row = [&](int dir, int x) {
-    int t2 = bx + (x + S / 2) % S;
-    if (t2 >= a.Px) t2 -= a.Px;
-    if (dir == 0) t2 = t2 + 1 == a.Px ? 0 : t2 + 1;
-    return t2;
-  };
-
-  float* gx = a.st_nobj + (size_t)b * N;
-  float* gy = a.st_nprobe + (size_t)b * N;
-  const float2* f0 = a.scratch_f + (size_t)b * M * N;
-  for (int m = 0; m < M; ++m) {
-    const float2* __restrict__ spec = a.probe_spec + (size_t)m * N;
-    for (int dir = 0; dir < 2; ++dir) {
-      // P_m shifted as in the forward pass
-#pragma unroll 1
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 sv[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) sv[i] = __ldg(spec + (fx0 + FXS * (c0 + i)) * S + fy);
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int x = fx0 + FXS * (c0 + i);
-          buf[x * LD + fy] = c_mul(sv[i], c_mul(rpx[x], rpy[fy]));
-        }
-      }
-      gsync();
-      inverse();
-      // times the moved object patch
-      const int oy = obj_col(dir);
-#pragma unroll 1
-      for (int c0 = 0; c0 < PER; c0 += CH) {
-        float2 ov[CH];
-#pragma unroll
-        for (int i = 0; i < CH; ++i) ov[i] = load_object(a, 0, obj_row(dir, ry0 + c0 + i), oy);
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-          const int idx = (ry0 + c0 + i) * LD + tg;
-          const float2 p = c_scale(buf[idx], invN);
-          buf[idx] = c_mul(p, ov[i]);
-        }
-      }
-      gsync();
-      forward();
-      float* gd = dir == 0 ? gx : gy;
-      for (int i = 0; i < PER; ++i) {
-        const int x = fx0 + FXS * i;
-        const int e = x * S + fy;
-        const float2 f = buf[x * LD + fy];
-        const float2 r = f0[(size_t)m * N + e];
-        const float2 d = c_sub(r, f);
-        const float v = 2.0f * __fadd_rn(__fmul_rn(d.x, r.x), __fmul_rn(d.y, r.y));
-        gd[e] = m == 0 ? v : gd[e] + v;
-      }
-    }
-  }
-
-  const float* amp = a.amplitudes + (size_t)arow * N;
-  const bool mixed = M > 1 || a.mixed_formula;
-  float sxx = 0.f, sxy = 0.f, syy = 0.f, sxd = 0.f, syd = 0.f;
-  for (int i = 0; i < PER; ++i) {
-    const int e = (fx0 + FXS * i) * S + fy;
-    float est;
-    if (mixed) {
-      float tt = 0.0f;
-      for (int m = 0; m < M; ++m) {
-        const float2 r = f0[(size_t)m * N + e];
-        const float av = hypotf(r.x, r.y);
-        tt += av * av;
-      }
-      const float amp_tot = sqrtf(tt);
-      est = amp_tot * amp_tot;
-    } else {
-      const float2 r = f0[e];
-      const float af = hypotf(r.x, r.y);
-      est = af * af;
-    }
-    const float A = amp[e];
-    const float d = __fsub_rn(__fmul_rn(A, A), est);
-    const float px = gx[e], py = gy[e];
-    sxx = fmaf(px, px, sxx);
-    sxy = fmaf(px, py, sxy);
-    syy = fmaf(py, py, syy);
-    sxd = fmaf(px, d, sxd);
-    syd = fmaf(py, d, syd);
-  }
-  double s5[5] = {sxx, sxy, syy, sxd, syd};
-  block_sum5<NT>(s5, red);
-  if (tid == 0) correction_update(a, prow, posx, posy, pos_ok, s5);
+// Square regions run the wave kernels (ptycho_wave.cuh) unless the batch needs
+// the general ones; at 128 x 128 the schedule setting can ask for those too.
+template <int SX, int SY>
+bool use_wave(const BatchArgs& a) {
+  const int schedule = get_schedule(SX);
+  return SX == SY && (schedule == 0 || schedule == 3) && wave_batch(a);
 }
 
 template <int SX, int SY, int NT>
 cudaError_t launch_correction_t(const BatchArgs& a, cudaStream_t s) {
   const size_t smem = Layout<SX, SY>::smem_bytes(false);
-  if constexpr (SX == 128 && SY == 128 && NT == 1024) {
-    const int schedule = get_schedule(128);
-    if (a.T == 1 && (schedule == 0 || schedule == 3)) {
-      const void* fn = reinterpret_cast<const void*>(position_correction_grouped_kernel<NT>);
-      const cudaError_t e0 = ensure_smem_limit(fn, (int)smem);
-      if (e0 != cudaSuccess) return e0;
-      position_correction_grouped_kernel<NT><<<a.B, NT, smem, s>>>(a);
-      return cudaGetLastError();
-    }
+  if constexpr (SX == SY) {
+    if (a.T == 1 && use_wave<SX, SY>(a)) return launch_wave_correction<SX>(a, s);
   }
   {
     const cudaError_t e0 =
@@ -1845,6 +1081,9 @@ cudaError_t launch_probe_inverse_t(const BatchArgs& a, cudaStream_t s) {
 
 template <int SX, int SY, int NT>
 cudaError_t launch_position_t(const BatchArgs& a, cudaStream_t s) {
+  if constexpr (SX == SY) {
+    if (use_wave<SX, SY>(a)) return launch_wave_position<SX>(a, s);
+  }
   const bool mixed_ms = a.T > 1 && a.M > 1;
   const bool mixed = (a.T == 1 && (a.M > 1 || a.mixed_formula)) || mixed_ms;
   const size_t smem = Layout<SX, SY>::smem_bytes(mixed);
@@ -1867,46 +1106,6 @@ cudaError_t launch_position_t(const BatchArgs& a, cudaStream_t s) {
                    : !plain ? 0
                    : a.T == 1 ? (a.M == 1 && !a.mixed_formula ? 1 : 2)
                    : 3;
-  if constexpr (SX == 128 && SY == 128 && NT == 1024) {
-    // the default (0) and schedule 3: passes by groups of warps
-    const int schedule = get_schedule(128);
-    // projection sets of one slice and probe without kept far fields
-    const bool ps1 = mode == 0 && a.projection && a.T == 1 && a.M == 1 && !a.mixed_formula &&
-                     !a.forward_only && !a.keep_farfield && !a.exact_probe_grad;
-    // mixed-state multislice gradient descent (its far fields are kept anyway)
-    const bool mms_gd = mode == 4 && !a.projection && !a.forward_only && !a.exact_probe_grad;
-    // single-slice single-probe gradient descent keeping its far fields
-    const bool keep1 = mode == 0 && !a.projection && a.keep_farfield && a.T == 1 && a.M == 1 &&
-                       !a.mixed_formula && !a.forward_only && !a.exact_probe_grad;
-    if ((mode == 1 || mode == 2 || mode == 3 || ps1 || mms_gd || keep1) &&
-        (schedule == 0 || schedule == 3)) {
-      const void* fn =
-          mode == 1   ? reinterpret_cast<const void*>(position_grouped_kernel<NT, 0>)
-          : mode == 3 ? reinterpret_cast<const void*>(position_grouped_kernel<NT, 1>)
-          : mode == 2 ? reinterpret_cast<const void*>(position_grouped_kernel<NT, 2>)
-          : mms_gd    ? reinterpret_cast<const void*>(position_grouped_kernel<NT, 4>)
-          : keep1     ? reinterpret_cast<const void*>(position_grouped_kernel<NT, 5>)
-                      : reinterpret_cast<const void*>(position_grouped_kernel<NT, 3>);
-      const cudaError_t e0 = ensure_smem_limit(fn, (int)smem);
-      if (e0 != cudaSuccess) return e0;
-      timing_before(s);
-      if (mode == 1)
-        position_grouped_kernel<NT, 0><<<a.B, NT, smem, s>>>(a);
-      else if (mode == 3)
-        position_grouped_kernel<NT, 1><<<a.B, NT, smem, s>>>(a);
-      else if (mode == 2)
-        position_grouped_kernel<NT, 2><<<a.B, NT, smem, s>>>(a);
-      else if (mms_gd)
-        position_grouped_kernel<NT, 4><<<a.B, NT, smem, s>>>(a);
-      else if (keep1)
-        position_grouped_kernel<NT, 5><<<a.B, NT, smem, s>>>(a);
-      else
-        position_grouped_kernel<NT, 3><<<a.B, NT, smem, s>>>(a);
-      const cudaError_t e1 = cudaGetLastError();
-      timing_after(s);
-      return e1;
-    }
-  }
   timing_before(s);
   switch (mode) {
     case 1: position_kernel<SX, SY, NT, 1><<<a.B, NT, smem, s>>>(a); break;
@@ -1930,6 +1129,12 @@ cudaError_t launch_position_t(const BatchArgs& a, cudaStream_t s) {
   namespace pty {                                                                        \
   cudaError_t launch_position_kernel_##NAME(const BatchArgs& a, cudaStream_t s) {        \
     return launch_position_t<SX, SY, NT>(a, s);                                          \
+  }                                                                                      \
+  int position_probe_rows_##NAME(const BatchArgs& a) {                                   \
+    if constexpr (SX == SY) {                                                            \
+      if (use_wave<SX, SY>(a)) return wave_gd_blocks<SX>(a);                             \
+    }                                                                                    \
+    return 0;                                                                            \
   }                                                                                      \
   cudaError_t launch_position_correction_##NAME(const BatchArgs& a, cudaStream_t s) {    \
     return launch_correction_t<SX, SY, NT>(a, s);                                        \

@@ -336,10 +336,15 @@ __global__ void __launch_bounds__(NT) probe_reduce_kernel(BatchArgs a) {
   if (e >= N) return;
   const float2* __restrict__ sp = a.st_probe;
   const float* __restrict__ snp = a.st_nprobe;
+  // rows of probe terms: one per position, or one per block of the resident
+  // position kernel
+  const int rows = a.probe_rows ? a.probe_rows : a.B;
+  const int rper = (rows + kProbeChunks - 1) / kProbeChunks;
+  const int rlo = c * rper, rhi = min(rows, rlo + rper);
   for (int m = 0; m < a.M; ++m) {
     float2 acc = make_float2(0.f, 0.f);
 #pragma unroll 8
-    for (int b = lo; b < hi; ++b) {
+    for (int b = rlo; b < rhi; ++b) {
       const float2 v = sp[((size_t)b * a.M + m) * N + e];
       acc.x += v.x;
       acc.y += v.y;
