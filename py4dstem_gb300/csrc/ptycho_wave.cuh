@@ -274,6 +274,59 @@ __device__ __forceinline__ void apply_mask(const WavePosition<S>& p, const float
   }
 }
 
+// Tensor memory as this thread's own storage: `words` consecutive 32-bit columns
+// of its lane (warp w owns lanes 32 (w % 4) .. + 31).
+__device__ __forceinline__ void tmem_put(uint32_t addr, const Cx2 (&v)[8]) {
+#define PTY_CELL(k)                                                                     \
+  "r"(__float_as_uint(v[k].re.x)), "r"(__float_as_uint(v[k].re.y)),                     \
+      "r"(__float_as_uint(v[k].im.x)), "r"(__float_as_uint(v[k].im.y))
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(
+          addr),
+      PTY_CELL(0), PTY_CELL(1), PTY_CELL(2), PTY_CELL(3), PTY_CELL(4), PTY_CELL(5), PTY_CELL(6),
+      PTY_CELL(7)
+      : "memory");
+#undef PTY_CELL
+}
+__device__ __forceinline__ void tmem_put(uint32_t addr, const float2 (&v)[8]) {
+#define PTY_TWO(k) "r"(__float_as_uint(v[k].x)), "r"(__float_as_uint(v[k].y))
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr),
+      PTY_TWO(0), PTY_TWO(1), PTY_TWO(2), PTY_TWO(3), PTY_TWO(4), PTY_TWO(5), PTY_TWO(6),
+      PTY_TWO(7)
+      : "memory");
+#undef PTY_TWO
+}
+// (the values arrive at tmem_wait_load)
+__device__ __forceinline__ void tmem_get(uint32_t addr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
+        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
+        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_load(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));  // uses stay below the wait
+}
+__device__ __forceinline__ void tmem_wait_store() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ Cx2 tmem_cell(const uint32_t (&r)[32], int k) {
+  return {make_float2(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1])),
+          make_float2(__uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]))};
+}
+
 // kKind 0: plain single-slice single-probe gradient descent; 1: any single-probe
 // model (multislice, projection sets, kept far fields, forward only, exact probe
 // gradient); 2: any mixed-state model (likewise).
@@ -287,15 +340,32 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_position_kernel(BatchArgs
   extern __shared__ float4 smem4[];
   __shared__ float red[W::NT / 32];
 
-  const int b = blockIdx.x;
   const int tid = threadIdx.x;
   const int T = kPlain ? 1 : a.T;
   const int M = kMixed ? a.M : 1;
-  const int prow = a.pos_rows ? a.pos_rows[b] : b;
-  const int arow = a.amp_rows ? a.amp_rows[b] : b;
   P p;
   p.carve(smem4);
   p.w.tables(tid);
+  // single-slice mixed states sum the modes' object terms and |P|^2 in tensor
+  // memory (48 words a task of this thread) and write them once
+  constexpr bool kTmem = kMixed && S == 128;
+  constexpr int WORDS = 48 * W::TITER;
+  __shared__ uint32_t tmem_base;
+  uint32_t tm = 0;
+  if constexpr (kTmem) {
+    if (p.w.warp == 0) nn::tmem_alloc(&tmem_base, 512);
+    nn::tc_fence_before();
+    __syncthreads();
+    nn::tc_fence_after();
+    tm = tmem_base + ((uint32_t)(p.w.warp & 3) << 21) + (p.w.warp >> 2) * WORDS;
+  }
+  const bool mode_sums = kTmem && T == 1 && M > 1;
+
+  // (resident blocks walk the batch where the launch has fewer blocks)
+#pragma unroll 1
+  for (int b = blockIdx.x; b < a.B; b += gridDim.x) {
+  const int prow = a.pos_rows ? a.pos_rows[b] : b;
+  const int arow = a.amp_rows ? a.amp_rows[b] : b;
   const float2 at = P::position(a, a.positions, b);
   const bool pos_ok = p.locate(a, at.x, at.y, 0);
   if (tid == 0) a.pos_round[b] = make_int2(p.x0, p.y0);
@@ -481,18 +551,54 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_position_kernel(BatchArgs
                 g.re = conj_mul(o[i], g).im;
                 g.im = make_float2(0.0f, 0.0f);
               }
-              float2 pn = abs2(pr[i]);
-              if (kMixed && m > 0) {
-                g = add(from_pair(ld_cell(gobj + e)), g);
-                pn = add2(ld_two(nobj + e), pn);
-              }
-              st_cell(gobj + e, to_pair(g));
-              st_two(nobj + e, pn);
+              const float2 pn = abs2(pr[i]);
               v[i] = conj_mul(o[i], chi);
               if (s == 0) {
                 if (!exact) st_cell(probe_term + e, to_pair(v[i]));
                 if (!kPlain && m == 0 && !a.nprobe_from_object)
                   st_two(a.st_nprobe + (size_t)b * N + e, abs2(o[i]));
+              }
+              if (mode_sums) {
+                pr[i] = g;  // summed below
+                o[i].re = pn;
+              } else if (kMixed && m > 0) {
+                st_cell(gobj + e, to_pair(add(from_pair(ld_cell(gobj + e)), g)));
+                st_two(nobj + e, add2(ld_two(nobj + e), pn));
+              } else {
+                st_cell(gobj + e, to_pair(g));
+                st_two(nobj + e, pn);
+              }
+            }
+            if constexpr (kTmem) {
+              if (mode_sums) {
+                const uint32_t tg = tm + 48 * it;
+                float2 pn[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) pn[i] = o[i].re;
+                if (m > 0) {
+                  uint32_t r[32];
+                  float q[16];
+                  tmem_get(tg, r);
+                  tmem_wait_load(r);
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) pr[i] = add(tmem_cell(r, i), pr[i]);
+                  nn::tmem_load16(tg + 32, q);
+#pragma unroll
+                  for (int i = 0; i < 8; ++i)
+                    pn[i] = add2(make_float2(q[2 * i], q[2 * i + 1]), pn[i]);
+                }
+                if (m + 1 < M) {
+                  tmem_put(tg, pr);
+                  tmem_put(tg + 32, pn);
+                  tmem_wait_store();
+                } else {
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) {
+                    const int e = p.real(t, i);
+                    st_cell(gobj + e, to_pair(pr[i]));
+                    st_two(nobj + e, pn[i]);
+                  }
+                }
               }
             }
           }
@@ -534,49 +640,14 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_position_kernel(BatchArgs
   }
   const float tot = block_sum<W::NT>(err + (err2.x + err2.y), red);
   if (tid == 0) a.err[b] = pos_ok ? tot : __int_as_float(0x7fc00000);
-}
-
-// Tensor memory as this thread's own storage: `words` consecutive 32-bit columns
-// of its lane (warp w owns lanes 32 (w % 4) .. + 31).
-__device__ __forceinline__ void tmem_put(uint32_t addr, const Cx2 (&v)[8]) {
-#define PTY_CELL(k)                                                                     \
-  "r"(__float_as_uint(v[k].re.x)), "r"(__float_as_uint(v[k].re.y)),                     \
-      "r"(__float_as_uint(v[k].im.x)), "r"(__float_as_uint(v[k].im.y))
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(
-          addr),
-      PTY_CELL(0), PTY_CELL(1), PTY_CELL(2), PTY_CELL(3), PTY_CELL(4), PTY_CELL(5), PTY_CELL(6),
-      PTY_CELL(7)
-      : "memory");
-#undef PTY_CELL
-}
-// (the values arrive at tmem_wait_load)
-__device__ __forceinline__ void tmem_get(uint32_t addr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(addr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_wait_load(uint32_t (&r)[32]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]));  // uses stay below the wait
-}
-__device__ __forceinline__ void tmem_wait_store() {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ Cx2 tmem_cell(const uint32_t (&r)[32], int k) {
-  return {make_float2(__uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1])),
-          make_float2(__uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]))};
+  __syncthreads();  // red and the ramps are rewritten by the next position
+  }
+  if constexpr (kTmem) {
+    nn::tc_fence_before();
+    __syncthreads();
+    nn::tc_fence_after();
+    if (p.w.warp == 0) nn::tmem_dealloc(tmem_base, 512);
+  }
 }
 
 // Plain single-slice single-probe gradient descent: one resident block per SM
@@ -933,22 +1004,26 @@ inline bool wave_plain(const BatchArgs& a) {
          !a.exact_probe_grad;
 }
 
-// Blocks of the resident gradient-descent kernel for this batch (the rows of
-// st_probe that hold probe terms), 0 when the batch runs one block per position.
-template <int S>
-int wave_gd_blocks(const BatchArgs& a) {
-  if (S != 128 || !wave_plain(a)) return 0;
+// One block per SM (its shared memory holds one wave of 128 x 128).
+inline int resident_blocks(int B) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 0;
-  return a.B < sms ? a.B : sms;
+  return B < sms ? B : sms;
+}
+
+// Blocks of the resident gradient-descent kernel for this batch (the rows of
+// st_probe that hold probe terms), 0 when the batch runs another kernel.
+template <int S>
+int wave_gd_blocks(const BatchArgs& a) {
+  return S == 128 && wave_plain(a) ? resident_blocks(a.B) : 0;
 }
 
 template <int S>
 cudaError_t launch_wave_position(const BatchArgs& a, cudaStream_t s) {
   using W = WaveFft<S>;
-  const int blocks = wave_gd_blocks<S>(a);
+  int blocks = wave_gd_blocks<S>(a);
   const size_t smem = blocks > 0 ? sizeof(float4) * WavePosition<S>::CELLS + 4 * S * (S + 8)
                                  : WavePosition<S>::smem_bytes(true);
   void (*fn)(BatchArgs) = wave_mixed(a) ? wave_position_kernel<S, 2> : wave_position_kernel<S, 1>;
@@ -961,6 +1036,7 @@ cudaError_t launch_wave_position(const BatchArgs& a, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   if ((e = launch_transmission(a, s)) != cudaSuccess) return e;
   timing_before(s);
+  if (S == 128 && blocks == 0 && wave_mixed(a)) blocks = resident_blocks(a.B);
   fn<<<blocks > 0 ? blocks : a.B, W::NT, smem, s>>>(a);
   e = cudaGetLastError();
   timing_after(s);

@@ -102,13 +102,10 @@ template <int DIR>
 __device__ __forceinline__ Cx2 twiddle(const Cx2& a, float2 w) {
   return twiddle<DIR>(a, make_float4(w.x, w.x, w.y, w.y));
 }
-// a times the constant c + DIR i s (s >= 0; one register pair per magnitude)
+// a times the constant c + DIR i s (c, s > 0; one register pair each)
 template <int DIR>
 __device__ __forceinline__ Cx2 rotate(const Cx2& a, float c, float s) {
-  const float2 re = c < 0.0f ? __fmul2_rn(neg2(a.re), dup(-c)) : __fmul2_rn(a.re, dup(c));
-  const float2 im = c < 0.0f ? __fmul2_rn(neg2(a.im), dup(-c)) : __fmul2_rn(a.im, dup(c));
-  return DIR < 0 ? Cx2{__ffma2_rn(a.im, dup(s), re), __ffma2_rn(neg2(a.re), dup(s), im)}
-                 : Cx2{__ffma2_rn(neg2(a.im), dup(s), re), __ffma2_rn(a.re, dup(s), im)};
+  return fma_i<DIR>(a, s, scale(a, c));
 }
 
 __device__ __forceinline__ Cx2 as_cx2(float4 v) {
@@ -128,7 +125,7 @@ __device__ __forceinline__ float4 to_pair(const Cx2& v) {
 constexpr float kSqrtHalf = 0.70710678118654752f;
 constexpr float kCos16 = 0.92387953251128674f;  // cos, sin of pi / 8
 constexpr float kSin16 = 0.38268343236508977f;
-constexpr float kSin60 = 0.86602540378443865f;
+constexpr double kSin60 = 0.86602540378443864676;  // sin of pi / 3
 
 // DFT of length 4 in place, natural order.
 template <int DIR>
@@ -152,13 +149,39 @@ __device__ __forceinline__ void dft4_w8(Cx2& a0, Cx2& a1, Cx2& a2, Cx2& a3) {
   a1 = fma_i<DIR>(d1, kSqrtHalf, d0);
   a3 = fma_i<-DIR>(d1, kSqrtHalf, d0);
 }
+// a sin(pi / 3), the factor as two floats: its float alone is a third of an ulp
+// off, the same way in every transform, which the sums over positions keep (the
+// probe of a 96 x 96 batch came out 10% further from float64 with it).
+__device__ __forceinline__ float2 times_sin60(float2 v) {
+  constexpr float hi = (float)kSin60, lo = (float)(kSin60 - (double)hi);
+  return __ffma2_rn(v, dup(hi), __fmul2_rn(v, dup(lo)));
+}
+__device__ __forceinline__ Cx2 times_sin60(const Cx2& a) {
+  return {times_sin60(a.re), times_sin60(a.im)};
+}
+// a exp(DIR i pi / 6) and a exp(DIR i pi / 3)
+template <int DIR>
+__device__ __forceinline__ Cx2 rotate30(const Cx2& a) {
+  return fma_i<DIR>(a, 0.5f, times_sin60(a));
+}
+template <int DIR>
+__device__ __forceinline__ Cx2 rotate60(const Cx2& a) {
+  const Cx2 u = times_sin60(a);
+  return fma_r(a, 0.5f, DIR < 0 ? Cx2{u.im, neg2(u.re)} : Cx2{neg2(u.im), u.re});
+}
+template <int DIR>
+__device__ __forceinline__ Cx2 rotate120(const Cx2& a) {
+  const Cx2 u = times_sin60(a);
+  return fms_r(a, 0.5f, DIR < 0 ? Cx2{u.im, neg2(u.re)} : Cx2{neg2(u.im), u.re});
+}
+
 template <int DIR>
 __device__ __forceinline__ void dft3(Cx2& a0, Cx2& a1, Cx2& a2) {
-  const Cx2 t = add(a1, a2), d = sub(a1, a2);
+  const Cx2 t = add(a1, a2), d = times_sin60(sub(a1, a2));
   const Cx2 m = fms_r(t, 0.5f, a0);
   a0 = add(a0, t);
-  a1 = fma_i<DIR>(d, kSin60, m);
-  a2 = fma_i<-DIR>(d, kSin60, m);
+  a1 = add_i<DIR>(m, d);
+  a2 = add_i<-DIR>(m, d);
 }
 
 // DFT of length R in place, natural order in and out.
@@ -222,10 +245,10 @@ __device__ __forceinline__ void dft_pair(Cx2 (&a)[R]) {
     // n = n2 + 4 n1 (n1 < 3), k = k1 + 3 k2
 #pragma unroll
     for (int n = 0; n < 4; ++n) dft3<DIR>(a[n], a[n + 4], a[n + 8]);
-    a[5] = rotate<DIR>(a[5], kSin60, 0.5f);
-    a[6] = rotate<DIR>(a[6], 0.5f, kSin60);
-    a[9] = rotate<DIR>(a[9], 0.5f, kSin60);
-    a[10] = rotate<DIR>(a[10], -0.5f, kSin60);
+    a[5] = rotate30<DIR>(a[5]);
+    a[6] = rotate60<DIR>(a[6]);
+    a[9] = rotate60<DIR>(a[9]);
+    a[10] = rotate120<DIR>(a[10]);
     dft4<DIR>(a[0], a[1], a[2], a[3]);
     {  // a7 carries the factor DIR i
       const Cx2 s0 = add(a[4], a[6]), d0 = sub(a[4], a[6]);
@@ -255,7 +278,7 @@ __device__ __forceinline__ void dft_pair(Cx2 (&a)[R]) {
     // n = n2 + 2 n1 (n1 < 3), k = k1 + 3 k2
     dft3<DIR>(a[0], a[2], a[4]);
     dft3<DIR>(a[1], a[3], a[5]);
-    const Cx2 w1 = rotate<DIR>(a[3], 0.5f, kSin60), w2 = rotate<DIR>(a[5], -0.5f, kSin60);
+    const Cx2 w1 = rotate60<DIR>(a[3]), w2 = rotate120<DIR>(a[5]);
     const Cx2 e0 = a[0], e1 = a[2], e2 = a[4], o0 = a[1];
     a[0] = add(e0, o0);
     a[3] = sub(e0, o0);
