@@ -3,13 +3,13 @@
 //
 // Object side (replaces _sum_overlapping_patches_bincounts, phase_base_class.py:1905-1968,
 // and the update lines of _gradient_descent_adjoint / _projection_sets_adjoint):
-//   object_reduce_kernel   one block per 16x16 object tile and slice. It lists, in
-//                          batch order, the positions whose patch touches the
-//                          tile; each warp sums every eighth list entry (a warp
-//                          load reads two whole staged tile rows), and the warp
-//                          partials are added in warp order (fixed, so the result
-//                          is deterministic); then the tile maximum of the
-//                          normaliser sums. Every staged value is read once.
+//   object_reduce_kernel   one or two blocks per 16x16 object tile and slice. Each
+//                          warp takes a part of the batch and sums the positions
+//                          whose patch touches the tile (a warp load reads two
+//                          whole staged tile rows); the warp partials are added
+//                          in warp order (fixed, so the result is deterministic);
+//                          then the tile maximum of the normaliser sums. Every
+//                          staged value is read once.
 //   object_update_kernel   N_O = 1/sqrt(1e-16 + ((1-m) S)^2 + (m max S)^2);
 //                          O += step G N_O (GD) or O = G N_O (projection sets).
 // Probe side: a chunked fixed-order sum over the batch, then the same
@@ -90,37 +90,56 @@ __device__ __forceinline__ void mark_nonfinite(const BatchArgs& a, float2 v) {
 }
 
 // ------------------------------------------------------------------ object side
-constexpr int kListChunk = 2048;
 constexpr int kRowsPerLane = 8;  // tile rows one lane visits per list entry (every other row)
 
-// One block (8 warps) per 16x16 object tile and slice. The block lists, in batch
-// order, the positions whose patch touches the tile (with the tile origin in
-// patch coordinates); warp w sums list entries w, w + 8, w + 16, ... For an
-// entry, lane l covers tile column l % 16 of rows l / 16, l / 16 + 2, ..., so
-// each warp load reads two whole 16-sample staged rows (two 128-byte lines of
-// the object term, two 64-byte ones of |P|^2) and the column arithmetic is paid
-// once per entry. The eight warp partials are then added in warp order for
-// each pixel (a fixed order: the result is deterministic), written as the
-// object gradient and normaliser sums, and the tile maximum of the normaliser
-// is taken. Every staged value is read once.
-__global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a) {
-  __shared__ int list[kListChunk];
-  __shared__ int list_d[kListChunk];  // (dx << 16) | dy: tile origin in patch coordinates
-  __shared__ int warp_count[NT / 32];
-  __shared__ int warp_base[NT / 32 + 1];
+// A cluster of C blocks (8 warps each) per 16x16 object tile and slice; warp w of
+// block r takes part 8 r + w of the batch. Its lanes test 32 positions at a time
+// for a patch that touches the tile (with the tile origin in patch coordinates)
+// and the warp then visits the hits in order. For a hit, lane l covers tile column
+// l % 16 of rows l / 16, l / 16 + 2, ..., so each warp load reads two whole
+// 16-sample staged rows (two 128-byte lines of the object term, two 64-byte ones of
+// |P|^2) and the column arithmetic is paid once per hit. The eight warp partials
+// are added in warp order for each pixel, then the blocks' sums in block order
+// through distributed shared memory (a fixed order: the result is deterministic),
+// written as the object gradient and normaliser sums, and the tile maximum of the
+// normaliser is taken. Every staged value is read once.
+// Bound: HBM and load latency (each warp keeps 16 loads in flight): 58 us per 1024
+// positions at 128 x 128 on a 319 x 319 object (3.5 TB/s), where a block-wide
+// list of the tile's positions took 99 us, with 8 warps waiting for the list's
+// barriers and one block a tile (up to 600 positions) running on alone.
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// the float at shared-memory address p of block `rank` of the cluster
+__device__ __forceinline__ float cluster_load(const float* p, uint32_t rank) {
+  uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(addr) : "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C) {
   __shared__ float part[NT / 32][3][NT];  // per-warp partials (g.x, g.y, n) per tile pixel
   __shared__ float red[NT / 32];
   static_assert(kTile * kTile == NT && kTile == 2 * kRowsPerLane, "tile layout");
   const int s = blockIdx.y;
   const int ntx = (a.Px + kTile - 1) / kTile;
   const int nty = (a.Py + kTile - 1) / kTile;
+  const int rank = C > 1 ? (int)cluster_rank() : 0;
+  const int index = blockIdx.x / C;
   // tile rows from the middle outwards (16, 15, 17, 14, ...): the scan sits in
   // the middle of the object, so the tiles with the longest lists start first
   // and the short ones at the edges fill the end of the launch
-  const int k = blockIdx.x / nty;
+  const int k = index / nty;
   const int mid = ntx / 2;
   const int trow = (k & 1) ? mid - ((k + 1) >> 1) : mid + (k >> 1);
-  const int tile = trow * nty + blockIdx.x % nty;
+  const int tile = trow * nty + index % nty;
   const int tx0 = trow * kTile;
   const int ty0 = (tile % nty) * kTile;
   const int tw = min(kTile, a.Px - tx0);
@@ -128,6 +147,9 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a) {
   const int N = a.Sx * a.Sy;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
+  const int parts = C * (NT / 32);
+  const int per = (a.B + parts - 1) / parts;
+  const int b0 = min(a.B, (rank * (NT / 32) + warp) * per), b1 = min(a.B, b0 + per);
 
   // staging axes: u is the slow one (rows), v the contiguous one
   const bool tr = a.staging_t != 0;
@@ -145,47 +167,30 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a) {
   const float* __restrict__ sn = a.st_nobj + (size_t)s * a.B * N;
   const int fminx = -(a.Sx / 2), fminy = -(a.Sy / 2);
 
-  for (int c0 = 0; c0 < a.B; c0 += kListChunk) {
-    const int cn = min(kListChunk, a.B - c0);
-    int count = 0;
-    // ordered compaction of the positions whose patch touches this tile
-    for (int base = 0; base < cn; base += NT) {
-      const int i = base + tid;
-      bool hit = false;
-      int dx = 0, dy = 0;
-      if (i < cn) {
-        const int2 r = a.pos_round[c0 + i];
-        dx = pmod(tx0 - (r.x + fminx), a.Px);
-        dy = pmod(ty0 - (r.y + fminy), a.Py);
-        hit = (dx < a.Sx || dx + tw - 1 >= a.Px) && (dy < a.Sy || dy + th - 1 >= a.Py);
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) warp_count[warp] = __popc(bal);
-      __syncthreads();
-      if (tid == 0) {
-        warp_base[0] = count;
-        for (int w = 0; w < NT / 32; ++w) warp_base[w + 1] = warp_base[w] + warp_count[w];
-      }
-      __syncthreads();
-      if (hit) {
-        const int slot = warp_base[warp] + __popc(bal & ((1u << lane) - 1u));
-        list[slot] = c0 + i;
-        list_d[slot] = (dx << 16) | dy;
-      }
-      count = warp_base[NT / 32];
-      __syncthreads();
+  for (int base = b0; base < b1; base += 32) {
+    const int i = base + lane;
+    bool hit = false;
+    int d = 0;  // (dx << 16) | dy
+    if (i < b1) {
+      const int2 r = a.pos_round[i];
+      const int dx = pmod(tx0 - (r.x + fminx), a.Px);
+      const int dy = pmod(ty0 - (r.y + fminy), a.Py);
+      hit = (dx < a.Sx || dx + tw - 1 >= a.Px) && (dy < a.Sy || dy + th - 1 >= a.Py);
+      d = (dx << 16) | dy;
     }
-    for (int l = warp; l < count; l += NT / 32) {
-      const int b = list[l];
-      const int d = list_d[l];
-      const int du = tr ? (d & 0xffff) : (d >> 16);
-      const int dv = tr ? (d >> 16) : (d & 0xffff);
+    unsigned hits = __ballot_sync(0xffffffffu, hit);
+    while (hits) {
+      const int bit = __ffs(hits) - 1;
+      hits &= hits - 1;
+      const int du0 = __shfl_sync(0xffffffffu, d, bit);
+      const int du = tr ? (du0 & 0xffff) : (du0 >> 16);
+      const int dv = tr ? (du0 >> 16) : (du0 & 0xffff);
       // this lane's column: patch coordinate sv (one object wrap at most)
       int sv = dv + iv;
       if (sv >= Pv) sv -= Pv;
       const bool vok = iv < tv && sv < Sv;
       const int lv = sv >= hv ? sv - hv : sv + hv;
-      const size_t col = (size_t)b * N + lv;
+      const size_t col = (size_t)(base + bit) * N + lv;
       float2 v[kRowsPerLane];
       float w[kRowsPerLane];
 #pragma unroll
@@ -209,7 +214,6 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a) {
         gn[k] += w[k];
       }
     }
-    __syncthreads();  // the list is rewritten by the next chunk
   }
 
   // warp partials in warp order, per tile pixel (u-major index iu * 16 + iv)
@@ -229,6 +233,22 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a) {
     g.y += part[w][1][tid];
     n += part[w][2][tid];
   }
+  if (C > 1) {
+    __syncthreads();
+    part[0][0][tid] = g.x;
+    part[0][1][tid] = g.y;
+    part[0][2][tid] = n;
+    cluster_sync();
+    if (rank == 0) {
+      for (int r = 1; r < C; ++r) {
+        g.x += cluster_load(&part[0][0][tid], r);
+        g.y += cluster_load(&part[0][1][tid], r);
+        n += cluster_load(&part[0][2][tid], r);
+      }
+    }
+    cluster_sync();  // the other blocks' sums have been read
+    if (rank != 0) return;
+  }
   const int pu = tid / kTile, pv = tid % kTile;
   const int px = tx0 + (tr ? pv : pu);
   const int py = ty0 + (tr ? pu : pv);
@@ -240,7 +260,28 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a) {
     m = n;
   }
   m = block_max(m, red);
-  if (tid == 0) a.tile_max[s * gridDim.x + tile] = m;
+  if (tid == 0) a.tile_max[s * (gridDim.x / C) + tile] = m;
+}
+
+// Two blocks a tile where one a tile would not fill the SMs' four block slots
+// (difference map of 4096 positions, 441 tiles: 3.21 -> 3.11 ms a pass; 96 x 96
+// scan, 196 tiles: 0.66 -> 0.64 ms) and each warp still has positions to test;
+// with 1024 tiles the second block costs 4% of the pass, and more blocks than two
+// were not faster anywhere (C = 1, 2, 4, 8 measured).
+cudaError_t launch_object_reduce(const BatchArgs& a, int ntiles, cudaStream_t s) {
+  const int C = ntiles * a.T <= 600 && a.B >= 128 ? 2 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ntiles * C, a.T);
+  cfg.blockDim = dim3(NT);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = C > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, object_reduce_kernel, a, C);
 }
 
 __global__ void __launch_bounds__(NT) object_update_kernel(BatchArgs a, int ntiles) {
@@ -876,7 +917,7 @@ cudaError_t launch_reduce_and_update(const BatchArgs& a, cudaStream_t s) {
     if (a.prepare_spectrum && (e = launch_probe_spectrum(a, fj.side)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(fj.join, fj.side)) != cudaSuccess) return e;
   }
-  object_reduce_kernel<<<dim3(ntiles, a.T), NT, 0, s>>>(a);
+  if ((e = launch_object_reduce(a, ntiles, s)) != cudaSuccess) return e;
   if (!a.fix_probe && a.nprobe_from_object &&
       (e = cudaStreamWaitEvent(s, fj.gathered, 0)) != cudaSuccess)
     return e;
@@ -1049,7 +1090,8 @@ cudaError_t launch_identical_slices(const BatchArgs& a, cudaStream_t s) {
 cudaError_t launch_overlap_accumulate(const BatchArgs& a, float* overlap, cudaStream_t s) {
   const int ntx = (a.Px + kTile - 1) / kTile;
   const int nty = (a.Py + kTile - 1) / kTile;
-  object_reduce_kernel<<<dim3(ntx * nty, 1), NT, 0, s>>>(a);
+  const cudaError_t e0 = launch_object_reduce(a, ntx * nty, s);
+  if (e0 != cudaSuccess) return e0;
   const size_t P = (size_t)a.Px * a.Py;
   overlap_accumulate_kernel<<<(unsigned)((P + NT - 1) / NT), NT, 0, s>>>(a, overlap);
   return cudaGetLastError();
@@ -1060,14 +1102,15 @@ cudaError_t launch_gradient(const BatchArgs& a, void* object_grad, float2* probe
   const int ntx = (a.Px + kTile - 1) / kTile;
   const int nty = (a.Py + kTile - 1) / kTile;
   const int ntiles = ntx * nty;
-  object_reduce_kernel<<<dim3(ntiles, a.T), NT, 0, s>>>(a);
+  cudaError_t e = launch_object_reduce(a, ntiles, s);
+  if (e != cudaSuccess) return e;
   if (probe_grad) {
     const int N = a.Sx * a.Sy;
     const int nb = (N + NT - 1) / NT;
     probe_reduce_kernel<<<dim3(nb, kProbeChunks), NT, 0, s>>>(a);
     probe_finalize_kernel<<<nb, NT, 0, s>>>(a);
     if (a.exact_probe_grad) {
-      cudaError_t e = launch_probe_inverse(a, s);
+      e = launch_probe_inverse(a, s);
       if (e != cudaSuccess) return e;
     }
   }
