@@ -981,6 +981,10 @@ __global__ void __launch_bounds__(NT, 1) probe_intensity_kernel(BatchArgs a) {
 
 template <int SX, int SY, int NT>
 cudaError_t launch_probe_intensity_t(const BatchArgs& a, cudaStream_t s) {
+  if constexpr (SX == SY) {
+    const int schedule = get_schedule(SX);
+    if (schedule == 0 || schedule == 3) return launch_wave_intensity<SX>(a, s);
+  }
   const size_t smem = Layout<SX, SY>::smem_bytes(false);
   {
     const cudaError_t e0 =

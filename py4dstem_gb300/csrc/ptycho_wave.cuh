@@ -983,6 +983,52 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
   if (tid == 0) correction_update(a, prow, posx, posy, pos_ok, s5);
 }
 
+// |P_b|^2 of the sub-pixel shifted probe (mode 0), as probe_intensity_kernel: the
+// first two phases of the position kernel.
+template <int S>
+__global__ void __launch_bounds__(WaveFft<S>::NT) wave_intensity_kernel(BatchArgs a) {
+  using W = WaveFft<S>;
+  using P = WavePosition<S>;
+  constexpr int N = W::N;
+  extern __shared__ float4 smem4[];
+  const int b = blockIdx.x;
+  P p;
+  p.carve(smem4);
+  p.w.tables(threadIdx.x);
+  const float2 at = P::position(a, a.positions, b);
+  p.locate(a, at.x, at.y, 0);
+  if (threadIdx.x == 0) a.pos_round[b] = make_int2(p.x0, p.y0);
+  __syncthreads();
+  const W& w = p.w;
+  const float invN = 1.0f / (float)N;
+#pragma unroll 1
+  for (int it = 0; it < W::TITER; ++it) {
+    const int t = w.lane + 32 * it;
+    if (W::TASKS % 32 != 0 && t >= W::TASKS) break;
+    Cx2 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = from_pair(ld_cell(a.probe_spec + p.fourier(t, i)));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = mul(v[i], p.ramp(t, i));
+    w.col_outer_store(t, v);
+  }
+  __syncwarp();
+  w.col_inner_inverse();
+  __syncthreads();
+  w.row_inner_inverse();
+  __syncwarp();
+  float* const dst = a.st_nobj + (size_t)b * N;
+#pragma unroll 1
+  for (int it = 0; it < W::TITER; ++it) {
+    const int t = w.lane + 32 * it;
+    if (W::TASKS % 32 != 0 && t >= W::TASKS) break;
+    Cx2 v[8];
+    w.row_outer_load(t, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) st_two(dst + p.real(t, i), abs2(scale(v[i], invN)));
+  }
+}
+
 // The wider loads and stores of these kernels need the caller's arrays aligned
 // (16-byte cells of the amplitudes, exit waves and propagators, float2 pairs of
 // the mask); a batch whose pointers are not takes the general kernel.
@@ -1041,6 +1087,16 @@ cudaError_t launch_wave_position(const BatchArgs& a, cudaStream_t s) {
   e = cudaGetLastError();
   timing_after(s);
   return e;
+}
+
+template <int S>
+cudaError_t launch_wave_intensity(const BatchArgs& a, cudaStream_t s) {
+  const size_t smem = WavePosition<S>::smem_bytes(false);
+  const cudaError_t e =
+      ensure_smem_limit(reinterpret_cast<const void*>(wave_intensity_kernel<S>), (int)smem);
+  if (e != cudaSuccess) return e;
+  wave_intensity_kernel<S><<<a.B, WaveFft<S>::NT, smem, s>>>(a);
+  return cudaGetLastError();
 }
 
 template <int S>
