@@ -4,7 +4,8 @@
 //
 // Activations are NHWC bfloat16 with a channel count that is a multiple of 8.
 // The 3 x 3 convolutions (stride 1, zero padding 1) are implicit GEMMs on the
-// tensor cores through tc_gemm_kernel (tc_gemm.cuh):
+// tensor cores, from halo tiles in shared memory (nn_conv_tile.cuh) or, for image
+// rows too wide for one, gathered by tc_gemm_kernel (tc_gemm.cuh):
 //   forward         y[p, co]   = sum_{tap, ci} x[p + off(tap), ci] w[co, tap, ci]
 //                   rows = pixels p, columns = co, K = 9 Cin
 //   input gradient  dx[p, ci]  = sum_{tap, co} dy[p - off(tap), co] wt[ci, tap, co]
@@ -19,6 +20,7 @@
 
 #include <cstdint>
 
+#include "nn_conv_tile.cuh"
 #include "nn_internal.h"
 #include "tc_gemm.cuh"
 
@@ -233,9 +235,63 @@ cudaError_t gemm_bf16(const bf16* a, const bf16* b, float* c, int M, int N, int 
                         StoreF32{c, M, N}, err, s);
 }
 
+// Tile shape of the rows kernel: columns a block (all of them up to 128) and 128-row
+// tiles a block, fewer of both while the launch would not give every SM a block;
+// smem 0 when a row of the image is too wide for a tile (the gathered GEMM then).
+struct RowsTile {
+  int BN, G;
+  size_t smem;
+};
+
+size_t rows_smem(int BN, int G, int pitch) {
+  const size_t P = tile_pixels(128 * G, pitch);
+  return 2 * (2 * P * 16 + 18 * (size_t)BN * 16) + 4 * P;
+}
+
+RowsTile rows_tile(const ConvLine& g, int N) {
+  RowsTile t{N <= 128 ? (N + 15) / 16 * 16 : 128, 4, 0};
+  auto blocks = [&] {
+    return ((g.Q + 128 * t.G - 1) / (128 * t.G)) * ((N + t.BN - 1) / t.BN);
+  };
+  while (t.G > 1 && (blocks() < 152 || t.G * t.BN > 256 ||
+                     rows_smem(t.BN, t.G, g.pitch) > 110 * 1024))
+    t.G /= 2;
+  while (t.BN > 32 && t.BN % 32 == 0 && blocks() < 152) t.BN /= 2;
+  const size_t need = rows_smem(t.BN, t.G, g.pitch);
+  t.smem = need <= 220 * 1024 ? need : 0;
+  return t;
+}
+
+template <class Epi>
+cudaError_t launch_rows(const bf16* x, const ConvLine& g, int C, const bf16* w, int N, int sign,
+                        const RowsTile& t, Epi epi, int* err, cudaStream_t s) {
+  auto kern = conv_rows_kernel<Epi>;
+  const cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(kern), (int)t.smem);
+  if (e != cudaSuccess) return e;
+  kern<<<dim3((g.Q + 128 * t.G - 1) / (128 * t.G), (N + t.BN - 1) / t.BN), kTileThreads, t.smem,
+         s>>>(x, g, C, w, N, t.BN, t.G, sign, epi, err);
+  return cudaGetLastError();
+}
+
+size_t wgrad_smem(int pitch) {
+  const size_t P = tile_pixels(kWgradPixels, pitch);
+  return kWgradRows / 8 * P * 16 + (size_t)kWgradColumns / 8 * kWgradPixels * 16 + 4 * P;
+}
+
+// the padded line of pixels has to fit an int index
+bool line_fits(int nb, int H, int W) {
+  return (size_t)nb * (H + 1) * (W + 1) < (size_t)1 << 30;
+}
+
 cudaError_t conv3x3_forward(const bf16* x, int nb, int H, int W, int cin, const bf16* w,
                             const float* bias, int cout, int relu, bf16* y, int* err,
                             cudaStream_t s) {
+  if (line_fits(nb, H, W)) {
+    const ConvLine g = conv_line(nb, H, W);
+    const RowsTile t = rows_tile(g, cout);
+    if (t.smem)
+      return launch_rows(x, g, cin, w, cout, 1, t, StoreActivation{y, bias, cout, relu}, err, s);
+  }
   const int M = nb * H * W;
   return launch_gemm_bn(pick_bn(cout), M, cout, 9 * cin, 1, 9 * cin,
                         Im2colFwd{x, nb, H, W, cin}, RowMajorBf16{w, cout, 9 * cin},
@@ -244,39 +300,88 @@ cudaError_t conv3x3_forward(const bf16* x, int nb, int H, int W, int cin, const 
 
 cudaError_t conv3x3_backward_data(const bf16* dy, int nb, int H, int W, int cout, const bf16* wt,
                                   int cin, float* dx, int* err, cudaStream_t s) {
+  if (line_fits(nb, H, W)) {
+    const ConvLine g = conv_line(nb, H, W);
+    const RowsTile t = rows_tile(g, cin);
+    if (t.smem)
+      return launch_rows(dy, g, cout, wt, cin, -1, t, StoreGradInput{dx, cin}, err, s);
+  }
   const int M = nb * H * W;
   return launch_gemm_bn(pick_bn(cin), M, cin, 9 * cout, 1, 9 * cout,
                         Im2colBwdData{dy, nb, H, W, cout}, RowMajorBf16{wt, cin, 9 * cout},
                         StoreGradInput{dx, cin}, err, s);
 }
 
-size_t conv3x3_wgrad_workspace(int nb, int H, int W, int cin, int cout) {
-  const int splits = wgrad_splits(nb * H * W);
-  return sizeof(float) * (size_t)splits * 9 * cin * cout;
-}
-
+// Parts of the weight gradient (K chunks): of at least 2048 pixels, at most 64 of
+// them, which any workspace holds; with room, one for every SM.
 int wgrad_splits(int npix) {
-  // K chunks of at least 2048 pixels (a multiple of the 64-element K stage), at
-  // most 64 of them
   int splits = (npix + 2047) / 2048;
   return splits > 64 ? 64 : (splits < 1 ? 1 : splits);
 }
 
+size_t conv3x3_wgrad_workspace_min(int nb, int H, int W, int cin, int cout) {
+  return sizeof(float) * (size_t)wgrad_splits(nb * H * W) * 9 * cin * cout;
+}
+
+size_t conv3x3_wgrad_workspace(int nb, int H, int W, int cin, int cout) {
+  const int tiles = (nb * (H + 1) * (W + 1) + kWgradPixels - 1) / kWgradPixels;
+  const int blocks = ((cin + kWgradRows - 1) / kWgradRows) *
+                     ((cout + kWgradColumns - 1) / kWgradColumns);
+  int splits = (152 + blocks - 1) / blocks;
+  if (splits > tiles) splits = tiles;
+  const size_t want = sizeof(float) * ((size_t)splits * 9 * cin * cout +
+                                       (size_t)kBiasBlocks * cout);
+  const size_t least = conv3x3_wgrad_workspace_min(nb, H, W, cin, cout);
+  return want > least ? want : least;
+}
+
 cudaError_t conv3x3_backward_weight(const bf16* x, const bf16* dy, int nb, int H, int W, int cin,
-                                    int cout, float* dw, float* db, float* part, int* err,
-                                    cudaStream_t s) {
+                                    int cout, float* dw, float* db, float* part,
+                                    size_t part_bytes, int* err, cudaStream_t s) {
   const int npix = nb * H * W;
-  const int splits = wgrad_splits(npix);
-  int kps = (npix + splits - 1) / splits;
-  kps = (kps + kBK - 1) / kBK * kBK;
   const int M = 9 * cin;
-  cudaError_t e = launch_gemm_bn(pick_bn(cout), M, cout, npix, splits, kps,
-                                 Im2colWgradA{x, nb, H, W, cin}, WgradB{dy, npix, cout},
-                                 StoreWgradPartial{part, M, cout}, err, s);
-  if (e != cudaSuccess) return e;
   const size_t n = (size_t)M * cout;
-  wgrad_reduce_kernel<<<(unsigned)((n + kEw - 1) / kEw), kEw, 0, s>>>(part, splits, n, dw);
-  if (db) bias_grad_kernel<<<cout, kEw, 0, s>>>(dy, npix, cout, db);
+  const size_t smem = wgrad_smem(W + 1);
+  // bias partials first, then as many weight parts as fit
+  const size_t bias_floats = (size_t)kBiasBlocks * cout;
+  const bool bias_parts = part_bytes / sizeof(float) >= bias_floats + n;
+  float* wpart = part + (bias_parts ? bias_floats : 0);
+  const size_t room = (part_bytes / sizeof(float) - (bias_parts ? bias_floats : 0)) / n;
+  int splits;
+  cudaError_t e;
+  if (line_fits(nb, H, W) && smem <= 220 * 1024) {
+    const ConvLine g = conv_line(nb, H, W);
+    const int tiles = (g.Q + kWgradPixels - 1) / kWgradPixels;
+    const int bm = (cin + kWgradRows - 1) / kWgradRows;
+    const int bn = (cout + kWgradColumns - 1) / kWgradColumns;
+    splits = (152 + bm * bn - 1) / (bm * bn);
+    if (splits > tiles) splits = tiles;
+    if ((size_t)splits > room) splits = (int)room;
+    if ((e = ensure_smem_limit(reinterpret_cast<const void*>(conv_wgrad_kernel), (int)smem)) !=
+        cudaSuccess)
+      return e;
+    conv_wgrad_kernel<<<dim3(splits, bm, bn), kTileThreads, smem, s>>>(x, dy, g, cin, cout, wpart,
+                                                                       err);
+    e = cudaGetLastError();
+  } else {
+    splits = wgrad_splits(npix);
+    if ((size_t)splits > room) splits = (int)room;
+    int kps = (npix + splits - 1) / splits;
+    kps = (kps + kBK - 1) / kBK * kBK;
+    e = launch_gemm_bn(pick_bn(cout), M, cout, npix, splits, kps, Im2colWgradA{x, nb, H, W, cin},
+                       WgradB{dy, npix, cout}, StoreWgradPartial{wpart, M, cout}, err, s);
+  }
+  if (e != cudaSuccess) return e;
+  wgrad_reduce_kernel<<<(unsigned)((n + kEw - 1) / kEw), kEw, 0, s>>>(wpart, splits, n, dw);
+  if (db) {
+    if (bias_parts) {
+      bias_partial_kernel<<<kBiasBlocks, kTileThreads, 0, s>>>(dy, npix, cout, part);
+      wgrad_reduce_kernel<<<(unsigned)((cout + kEw - 1) / kEw), kEw, 0, s>>>(part, kBiasBlocks,
+                                                                             cout, db);
+    } else {
+      bias_grad_kernel<<<cout, kEw, 0, s>>>(dy, npix, cout, db);
+    }
+  }
   return cudaGetLastError();
 }
 
@@ -344,12 +449,13 @@ int ptycho_nn_conv3x3_backward_weight(const void* x, const void* dy, int32_t bat
   if (!x || !dy || !dweight || !workspace || !err_flag ||
       !conv_shape_ok(batch, height, width, cin, cout))
     return PTYCHO_ERR_INVALID_ARGUMENT;
-  if (workspace_bytes < pty::nn::conv3x3_wgrad_workspace(batch, height, width, cin, cout))
+  if (workspace_bytes < pty::nn::conv3x3_wgrad_workspace_min(batch, height, width, cin, cout))
     return PTYCHO_ERR_WORKSPACE;
   using pty::nn::bf16;
   cudaError_t e = pty::nn::conv3x3_backward_weight(
       static_cast<const bf16*>(x), static_cast<const bf16*>(dy), batch, height, width, cin, cout,
-      dweight, dbias, static_cast<float*>(workspace), err_flag, static_cast<cudaStream_t>(stream));
+      dweight, dbias, static_cast<float*>(workspace), workspace_bytes, err_flag,
+      static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_CUDA;
 }
 

@@ -29,11 +29,12 @@ cudaError_t conv3x3_forward(const bf16* x, int nb, int H, int W, int cin, const 
                             cudaStream_t s);
 cudaError_t conv3x3_backward_data(const bf16* dy, int nb, int H, int W, int cout, const bf16* wt,
                                   int cin, float* dx, int* err, cudaStream_t s);
-int wgrad_splits(int npix);
+// part: the workspace; the size that fills the GPU, and the least that is taken.
 size_t conv3x3_wgrad_workspace(int nb, int H, int W, int cin, int cout);
+size_t conv3x3_wgrad_workspace_min(int nb, int H, int W, int cin, int cout);
 cudaError_t conv3x3_backward_weight(const bf16* x, const bf16* dy, int nb, int H, int W, int cin,
-                                    int cout, float* dw, float* db, float* part, int* err,
-                                    cudaStream_t s);
+                                    int cout, float* dw, float* db, float* part,
+                                    size_t part_bytes, int* err, cudaStream_t s);
 
 }  // namespace nn
 }  // namespace pty

@@ -483,7 +483,10 @@ struct Net {
   cudaError_t conv_back(int l, const bf16* x, const bf16* g, float* dx) {
     cudaError_t e = conv3x3_backward_weight(x, g, nb, hl(l), wl(l), kCin[l], kCout[l],
                                             p<float>(pl.gw[l]), p<float>(pl.gb[l]),
-                                            a<float>(al.wpart), err, s);
+                                            a<float>(al.wpart),
+                                            conv3x3_wgrad_workspace(nb, hl(l), wl(l), kCin[l],
+                                                                    kCout[l]),
+                                            err, s);
     if (e != cudaSuccess || !dx) return e;
     return conv3x3_backward_data(g, nb, hl(l), wl(l), kCout[l], p<bf16>(pl.wt16[l]), kCin[l],
                                  dx, err, s);
