@@ -134,6 +134,7 @@ struct WgradB {  // rows = co, K = pixels: dy[p, co] for 8 consecutive pixels
 };
 
 struct StoreActivation {  // y[p, co] = bf16(act(v + bias[co])), Cout a multiple of 16
+  static constexpr bool kWarp = false;
   bf16* y;
   const float* bias;
   int Cout, relu;
@@ -154,10 +155,48 @@ struct StoreActivation {  // y[p, co] = bf16(act(v + bias[co])), Cout a multiple
 struct StoreGradInput {  // dx[p, ci] (float), columns beyond Cin dropped
   float* dx;
   int Cin;
-  __device__ void operator()(int r, int c0, const float (&v)[16], int) const {
+  bool whole;  // rows start on 16 bytes
+  static constexpr bool kWarp = true;
+  // a warp's 32 rows of 16 columns through shared memory, so that four lanes
+  // write the 64 bytes of a row together (32 rows of 16 bytes each otherwise)
+  __device__ void store(float* buf, int lane, int pixel, int c0, const float (&v)[16]) const {
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (c0 + i < Cin) dx[(size_t)r * Cin + c0 + i] = v[i];
+    for (int i = 0; i < 16; i += 4)
+      *reinterpret_cast<float4*>(buf + lane * kEpiPitch + i) =
+          make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    __syncwarp();
+    const int c = 4 * (lane & 3);
+#pragma unroll
+    for (int r = 0; r < 32; r += 8) {
+      const int row = r + (lane >> 2);
+      const int px = __shfl_sync(0xffffffffu, pixel, row);
+      const float4 u = *reinterpret_cast<const float4*>(buf + row * kEpiPitch + c);
+      if (px >= 0 && c0 + c < Cin) {
+        float* dst = dx + (size_t)px * Cin + c0 + c;
+        if (whole) {
+          *reinterpret_cast<float4*>(dst) = u;
+        } else {  // (Cin is a multiple of 8)
+          dst[0] = u.x;
+          dst[1] = u.y;
+          dst[2] = u.z;
+          dst[3] = u.w;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  __device__ void operator()(int r, int c0, const float (&v)[16], int) const {
+    float* dst = dx + (size_t)r * Cin + c0;
+    if (whole) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4)
+        if (c0 + i < Cin)
+          *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (c0 + i < Cin) dst[i] = v[i];
+    }
   }
 };
 
@@ -207,6 +246,7 @@ __global__ void wgrad_reduce_kernel(const float* part, int splits, size_t n, flo
   const size_t i = (size_t)blockIdx.x * kEw + threadIdx.x;
   if (i >= n) return;
   float s = 0.0f;
+#pragma unroll 16  // (the loads of 16 parts in flight, the sum in order)
   for (int z = 0; z < splits; ++z) s += part[(size_t)z * n + i];
   dw[i] = s;
 }
@@ -239,26 +279,28 @@ cudaError_t gemm_bf16(const bf16* a, const bf16* b, float* c, int M, int N, int 
 // tiles a block, fewer of both while the launch would not give every SM a block;
 // smem 0 when a row of the image is too wide for a tile (the gathered GEMM then).
 struct RowsTile {
-  int BN, G;
+  int BN, G, buffers;
   size_t smem;
 };
 
-size_t rows_smem(int BN, int G, int pitch) {
+size_t rows_smem(int BN, int G, int pitch, int buffers) {
   const size_t P = tile_pixels(128 * G, pitch);
-  return 2 * (2 * P * 16 + 18 * (size_t)BN * 16) + 4 * P;
+  const size_t need = buffers * (2 * P * 16 + 18 * (size_t)BN * 16) + 4 * P;
+  const size_t epilogue = sizeof(float) * kTileThreads * kEpiPitch;
+  return need > epilogue ? need : epilogue;
 }
 
-RowsTile rows_tile(const ConvLine& g, int N) {
-  RowsTile t{N <= 128 ? (N + 15) / 16 * 16 : 128, 4, 0};
+RowsTile rows_tile(const ConvLine& g, int C, int N) {
+  const int stages = (C + kStageChannels - 1) / kStageChannels;
+  RowsTile t{N <= 128 ? (N + 15) / 16 * 16 : 128, 4, stages < 3 ? (stages < 2 ? 2 : stages) : 3, 0};
   auto blocks = [&] {
     return ((g.Q + 128 * t.G - 1) / (128 * t.G)) * ((N + t.BN - 1) / t.BN);
   };
-  while (t.G > 1 && (blocks() < 152 || t.G * t.BN > 256 ||
-                     rows_smem(t.BN, t.G, g.pitch) > 110 * 1024))
-    t.G /= 2;
+  auto smem = [&] { return rows_smem(t.BN, t.G, g.pitch, t.buffers); };
+  while (t.G > 1 && (blocks() < 152 || t.G * t.BN > 256 || smem() > 110 * 1024)) t.G /= 2;
   while (t.BN > 32 && t.BN % 32 == 0 && blocks() < 152) t.BN /= 2;
-  const size_t need = rows_smem(t.BN, t.G, g.pitch);
-  t.smem = need <= 220 * 1024 ? need : 0;
+  if (smem() > 220 * 1024) t.buffers = 2;
+  t.smem = smem() <= 220 * 1024 ? smem() : 0;
   return t;
 }
 
@@ -269,13 +311,14 @@ cudaError_t launch_rows(const bf16* x, const ConvLine& g, int C, const bf16* w, 
   const cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(kern), (int)t.smem);
   if (e != cudaSuccess) return e;
   kern<<<dim3((g.Q + 128 * t.G - 1) / (128 * t.G), (N + t.BN - 1) / t.BN), kTileThreads, t.smem,
-         s>>>(x, g, C, w, N, t.BN, t.G, sign, epi, err);
+         s>>>(x, g, C, w, N, t.BN, t.G, t.buffers, sign, epi, err);
   return cudaGetLastError();
 }
 
-size_t wgrad_smem(int pitch) {
-  const size_t P = tile_pixels(kWgradPixels, pitch);
-  return kWgradRows / 8 * P * 16 + (size_t)kWgradColumns / 8 * kWgradPixels * 16 + 4 * P;
+size_t wgrad_smem(int pitch, int buffers) {
+  const size_t P = wgrad_pixels(kWgradPixels, pitch);
+  return buffers * (kWgradRows / 8 * P * 16 + (size_t)kWgradColumns / 8 * kWgradPixels * 16) +
+         4 * P;
 }
 
 // the padded line of pixels has to fit an int index
@@ -288,7 +331,7 @@ cudaError_t conv3x3_forward(const bf16* x, int nb, int H, int W, int cin, const 
                             cudaStream_t s) {
   if (line_fits(nb, H, W)) {
     const ConvLine g = conv_line(nb, H, W);
-    const RowsTile t = rows_tile(g, cout);
+    const RowsTile t = rows_tile(g, cin, cout);
     if (t.smem)
       return launch_rows(x, g, cin, w, cout, 1, t, StoreActivation{y, bias, cout, relu}, err, s);
   }
@@ -300,16 +343,17 @@ cudaError_t conv3x3_forward(const bf16* x, int nb, int H, int W, int cin, const 
 
 cudaError_t conv3x3_backward_data(const bf16* dy, int nb, int H, int W, int cout, const bf16* wt,
                                   int cin, float* dx, int* err, cudaStream_t s) {
+  const bool whole = cin % 4 == 0 && reinterpret_cast<uintptr_t>(dx) % 16 == 0;
   if (line_fits(nb, H, W)) {
     const ConvLine g = conv_line(nb, H, W);
-    const RowsTile t = rows_tile(g, cin);
+    const RowsTile t = rows_tile(g, cout, cin);
     if (t.smem)
-      return launch_rows(dy, g, cout, wt, cin, -1, t, StoreGradInput{dx, cin}, err, s);
+      return launch_rows(dy, g, cout, wt, cin, -1, t, StoreGradInput{dx, cin, whole}, err, s);
   }
   const int M = nb * H * W;
   return launch_gemm_bn(pick_bn(cin), M, cin, 9 * cout, 1, 9 * cout,
                         Im2colBwdData{dy, nb, H, W, cout}, RowMajorBf16{wt, cin, 9 * cout},
-                        StoreGradInput{dx, cin}, err, s);
+                        StoreGradInput{dx, cin, whole}, err, s);
 }
 
 // Parts of the weight gradient (K chunks): of at least 2048 pixels, at most 64 of
@@ -341,7 +385,8 @@ cudaError_t conv3x3_backward_weight(const bf16* x, const bf16* dy, int nb, int H
   const int npix = nb * H * W;
   const int M = 9 * cin;
   const size_t n = (size_t)M * cout;
-  const size_t smem = wgrad_smem(W + 1);
+  const int buffers = wgrad_smem(W + 1, 2) <= 220 * 1024 ? 2 : 1;
+  const size_t smem = wgrad_smem(W + 1, buffers);
   // bias partials first, then as many weight parts as fit
   const size_t bias_floats = (size_t)kBiasBlocks * cout;
   const bool bias_parts = part_bytes / sizeof(float) >= bias_floats + n;
@@ -360,8 +405,8 @@ cudaError_t conv3x3_backward_weight(const bf16* x, const bf16* dy, int nb, int H
     if ((e = ensure_smem_limit(reinterpret_cast<const void*>(conv_wgrad_kernel), (int)smem)) !=
         cudaSuccess)
       return e;
-    conv_wgrad_kernel<<<dim3(splits, bm, bn), kTileThreads, smem, s>>>(x, dy, g, cin, cout, wpart,
-                                                                       err);
+    conv_wgrad_kernel<<<dim3(splits, bm, bn), kTileThreads, smem, s>>>(x, dy, g, cin, cout, buffers,
+                                                                       wpart, err);
     e = cudaGetLastError();
   } else {
     splits = wgrad_splits(npix);
