@@ -260,9 +260,9 @@ __device__ __forceinline__ float2 cis_rounded(float phi) {
   }
   const DF x{phi, 0.0f};
   const DF x2 = df_mul(x, x);
-  // the terms from n = 7 on are below 2^-30 (sine) and 2^-26 (cosine): single
+  // the terms from n = 8 on are below 2^-37 (sine) and 2^-33 (cosine): single
   // floats carry them without moving a rounded result
-  constexpr int kSingle = 7;
+  constexpr int kSingle = 8;
   float sf = kCoefs.shi[11], cf = kCoefs.chi[11];
 #pragma unroll
   for (int n = 10; n >= kSingle; --n) {

@@ -891,7 +891,7 @@ namespace {
 template <int SX, int SY>
 bool use_wave(const BatchArgs& a) {
   const int schedule = get_schedule(SX);
-  return SX == SY && (schedule == 0 || schedule == 3) && wave_batch(a);
+  return SX == SY && (schedule == 0 || schedule == 3) && !small_batch(a) && wave_batch(a);
 }
 
 template <int SX, int SY, int NT>

@@ -93,7 +93,8 @@ __device__ __forceinline__ void mark_nonfinite(const BatchArgs& a, float2 v) {
 constexpr int kRowsPerLane = 8;  // tile rows one lane visits per list entry (every other row)
 
 // A cluster of C blocks (8 warps each) per 16x16 object tile and slice; warp w of
-// block r takes part 8 r + w of the batch. Its lanes test 32 positions at a time
+// block r takes part 8 r + w of the batch or, for small batches (in_turn, C = 1),
+// every eighth of the positions that touch the tile. Its lanes test 32 positions at a time
 // for a patch that touches the tile (with the tile origin in patch coordinates)
 // and the warp then visits the hits in order. For a hit, lane l covers tile column
 // l % 16 of rows l / 16, l / 16 + 2, ..., so each warp load reads two whole
@@ -124,7 +125,19 @@ __device__ __forceinline__ float cluster_load(const float* p, uint32_t rank) {
   return v;
 }
 
-__global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C) {
+__device__ __forceinline__ float2 cluster_load2(const float2* p, uint32_t rank) {
+  uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
+  float2 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(addr) : "r"(rank));
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];"
+               : "=f"(v.x), "=f"(v.y)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C,
+                                                             int in_turn) {
   __shared__ float part[NT / 32][3][NT];  // per-warp partials (g.x, g.y, n) per tile pixel
   __shared__ float red[NT / 32];
   static_assert(kTile * kTile == NT && kTile == 2 * kRowsPerLane, "tile layout");
@@ -149,7 +162,9 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C
   const int lane = tid & 31, warp = tid >> 5;
   const int parts = C * (NT / 32);
   const int per = (a.B + parts - 1) / parts;
-  const int b0 = min(a.B, (rank * (NT / 32) + warp) * per), b1 = min(a.B, b0 + per);
+  const int b0 = in_turn ? 0 : min(a.B, (rank * (NT / 32) + warp) * per);
+  const int b1 = in_turn ? a.B : min(a.B, b0 + per);
+  int turn = 0;  // the next hit's place among the tile's
 
   // staging axes: u is the slow one (rows), v the contiguous one
   const bool tr = a.staging_t != 0;
@@ -179,6 +194,11 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C
       d = (dx << 16) | dy;
     }
     unsigned hits = __ballot_sync(0xffffffffu, hit);
+    if (in_turn) {
+      const int place = turn + __popc(hits & ((1u << lane) - 1u));
+      turn += __popc(hits);
+      hits = __ballot_sync(0xffffffffu, hit && place % (NT / 32) == warp);
+    }
     while (hits) {
       const int bit = __ffs(hits) - 1;
       hits &= hits - 1;
@@ -269,7 +289,9 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C
 // with 1024 tiles the second block costs 4% of the pass, and more blocks than two
 // were not faster anywhere (C = 1, 2, 4, 8 measured).
 cudaError_t launch_object_reduce(const BatchArgs& a, int ntiles, cudaStream_t s) {
-  const int C = ntiles * a.T <= 600 && a.B >= 128 ? 2 : 1;
+  const bool small = small_batch(a);
+  const int C = ntiles * a.T <= 600 && a.B >= 128 && !small ? 2 : 1;
+  const int in_turn = small;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ntiles * C, a.T);
   cfg.blockDim = dim3(NT);
@@ -281,7 +303,7 @@ cudaError_t launch_object_reduce(const BatchArgs& a, int ntiles, cudaStream_t s)
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = C > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, object_reduce_kernel, a, C);
+  return cudaLaunchKernelEx(&cfg, object_reduce_kernel, a, C, in_turn);
 }
 
 __global__ void __launch_bounds__(NT) object_update_kernel(BatchArgs a, int ntiles) {
@@ -482,6 +504,158 @@ __global__ void __launch_bounds__(NT) probe_update_kernel(BatchArgs a, int nbloc
     }
     mark_nonfinite(a, a.probe[o]);
   }
+}
+
+// The rest of the probe side for square probes in one launch: a cluster of eight
+// blocks per mode. Block r owns S / 8 rows: it adds the chunk partials (the order
+// of probe_finalize_kernel), the cluster shares the normaliser maximum, the rows
+// are updated (the expressions of probe_update_kernel) and, for the next batch,
+// transformed: rows in the block, then columns gathered from the other blocks'
+// shared memory (the passes and twiddles of the staged line transforms, so the
+// same bits). Bound: latency. It takes the place of four launches on the probe side's
+// chain: 64 x 64, batch 64: 45.2 -> 41.6 us a batch; 96 x 96 scan of 1763 positions:
+// 641 -> 609 us a pass; four modes at 128 x 128: 3.83 -> 3.75 ms a pass.
+constexpr int kFinishBlocks = 8;
+constexpr int kFinishThreads = 512;
+
+template <int S>
+__global__ void __launch_bounds__(kFinishThreads) probe_finish_kernel(BatchArgs a) {
+  constexpr int LINES = S / kFinishBlocks;
+  constexpr int LD = S + 1;
+  constexpr int N = S * S;
+  constexpr int PX = LINES * S;  // pixels of a block
+  constexpr int PER = (PX + kFinishThreads - 1) / kFinishThreads;
+  extern __shared__ float2 finish_smem[];
+  float2* const rows = finish_smem;             // LINES x LD
+  float2* const cols = rows + LINES * LD;       // LINES x LD
+  float2* const tw = cols + LINES * LD;         // S
+  __shared__ float red[kFinishThreads / 32];
+  __shared__ float block_value;
+  const int m = blockIdx.x / kFinishBlocks;
+  const int rank = (int)cluster_rank();
+  const int tid = threadIdx.x;
+  const int e0 = rank * PX;
+  if (a.prepare_spectrum) fill_twiddles<S, kFinishThreads>(tw);
+
+  float nrm[PER];
+  float mx = 0.0f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int k = tid + i * kFinishThreads;
+    float n = 0.0f;
+    if (PX % kFinishThreads == 0 || k < PX) {
+#pragma unroll
+      for (int c = 0; c < kProbeChunks; ++c) n += a.probe_npart[(size_t)c * N + e0 + k];
+      mx = fmaxf(mx, n);
+    }
+    nrm[i] = n;
+  }
+  mx = warp_max(mx);
+  if ((tid & 31) == 0) red[tid >> 5] = mx;
+  __syncthreads();
+  if (tid < 32) {
+    const float t = warp_max(tid < kFinishThreads / 32 ? red[tid] : 0.0f);
+    if (tid == 0) block_value = t;
+  }
+  cluster_sync();
+  float smax = 0.0f;
+#pragma unroll
+  for (int r = 0; r < kFinishBlocks; ++r) smax = fmaxf(smax, cluster_load(&block_value, r));
+
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int k = tid + i * kFinishThreads;
+    if (PX % kFinishThreads != 0 && k >= PX) break;
+    float2 g = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < kProbeChunks; ++c) {
+      const float2 v = a.probe_part[((size_t)c * a.M + m) * N + e0 + k];
+      g.x += v.x;
+      g.y += v.y;
+    }
+    const float q = normaliser(nrm[i], smax, a.norm_min);
+    const size_t o = (size_t)m * N + e0 + k;
+    float2 r;
+    if (a.projection) {
+      r = make_float2(__fmul_rn(g.x, q), __fmul_rn(g.y, q));
+    } else {
+      float2 u;
+      if (a.T > 1) {
+        u = make_float2(__fmul_rn(__fmul_rn(a.step, g.x), q), __fmul_rn(__fmul_rn(a.step, g.y), q));
+      } else {
+        u = make_float2(__fmul_rn(a.step, __fmul_rn(g.x, q)), __fmul_rn(a.step, __fmul_rn(g.y, q)));
+      }
+      const float2 v = a.probe[o];
+      r = make_float2(__fadd_rn(v.x, u.x), __fadd_rn(v.y, u.y));
+    }
+    a.probe[o] = r;
+    mark_nonfinite(a, r);
+    rows[k / S * LD + k % S] = r;
+  }
+  if (!a.prepare_spectrum) {
+    cluster_sync();  // every block has read the others' maxima
+    return;
+  }
+  __syncthreads();
+  Schedule<S>::template run<LINES, kFinishThreads, -1>(rows, LD, 1, tw, tid);
+  cluster_sync();
+  // cols[l][x] = row x, column e0 / S + l, from the block that owns row x
+  for (int k = tid; k < PX; k += kFinishThreads) {
+    const int x = k / LINES, l = k % LINES;
+    cols[l * LD + x] = cluster_load2(rows + x % LINES * LD + rank * LINES + l, x / LINES);
+  }
+  cluster_sync();  // (also the last access to the other blocks' shared memory)
+  Schedule<S>::template run<LINES, kFinishThreads, -1>(cols, LD, 1, tw, tid);
+  float2* const spec = a.probe_spec + (size_t)m * N;
+  for (int k = tid; k < PX; k += kFinishThreads) {
+    const int x = k / LINES, l = k % LINES;
+    spec[(size_t)x * S + rank * LINES + l] = cols[l * LD + x];
+  }
+  if (blockIdx.x == 0)  // the tables that the general position kernels read
+    for (int i = tid; i < S; i += kFinishThreads) a.tw[i] = a.tw[S + i] = tw[i];
+}
+
+template <int S>
+cudaError_t launch_probe_finish_t(const BatchArgs& a, cudaStream_t s) {
+  const size_t smem = sizeof(float2) * (2 * (size_t)(S / kFinishBlocks) * (S + 1) + S);
+  cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(probe_finish_kernel<S>),
+                                    (int)smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kFinishBlocks * a.M);
+  cfg.blockDim = dim3(kFinishThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kFinishBlocks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, probe_finish_kernel<S>, a);
+}
+
+// The probe side after probe_reduce_kernel: the sums, the update and, with
+// prepare_spectrum, the next batch's spectrum. Probes that are not square (and
+// the transposed staging of the register-resident kernel) take one kernel a step.
+cudaError_t launch_probe_finish(const BatchArgs& a, cudaStream_t s) {
+  if (a.Sx == a.Sy && !a.staging_t) {
+    switch (a.Sx) {
+      case 32: return launch_probe_finish_t<32>(a, s);
+      case 48: return launch_probe_finish_t<48>(a, s);
+      case 64: return launch_probe_finish_t<64>(a, s);
+      case 96: return launch_probe_finish_t<96>(a, s);
+      case 128: return launch_probe_finish_t<128>(a, s);
+      case 256: return launch_probe_finish_t<256>(a, s);
+      default: break;
+    }
+  }
+  const int nb = (a.Sx * a.Sy + NT - 1) / NT;
+  probe_finalize_kernel<<<nb, NT, 0, s>>>(a);
+  probe_update_kernel<<<nb, NT, 0, s>>>(a, nb);
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess || !a.prepare_spectrum ? e : launch_probe_spectrum(a, s);
 }
 
 // ------------------------------------------------------------- gradient export
@@ -910,11 +1084,8 @@ cudaError_t launch_reduce_and_update(const BatchArgs& a, cudaStream_t s) {
     // update below rewrites: the update waits for it
     if (a.nprobe_from_object && (e = cudaEventRecord(fj.gathered, fj.side)) != cudaSuccess)
       return e;
-    probe_finalize_kernel<<<nb, NT, 0, fj.side>>>(a);
-    probe_update_kernel<<<nb, NT, 0, fj.side>>>(a, nb);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // the next batch's spectrum of the updated probe, off the critical path
-    if (a.prepare_spectrum && (e = launch_probe_spectrum(a, fj.side)) != cudaSuccess) return e;
+    if ((e = launch_probe_finish(a, fj.side)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(fj.join, fj.side)) != cudaSuccess) return e;
   }
   if ((e = launch_object_reduce(a, ntiles, s)) != cudaSuccess) return e;
