@@ -295,6 +295,7 @@ static int run_batch(const ptycho_geometry* g, void* object, void* probe,
                              ? 1
                              : 0;
   a.probe_rows = a.staging_t ? 0 : position_probe_rows(a);
+  if (a.probe_rows) a.nprobe_from_object = 1;  // (the resident kernel stages none)
   e = a.staging_t ? launch_position_v2(a, s) : launch_position_kernel(a, s);
   if (e != cudaSuccess) return cuda_fail(e, "position kernel");
   e = launch_reduce_and_update(a, s);

@@ -661,7 +661,12 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_position_kernel(BatchArgs
 // blockIdx.x of st_probe (probe_reduce_kernel then adds gridDim.x rows instead
 // of B). Positions go to blocks by index, so every sum has a fixed order. The
 // next position's amplitudes and ramps are fetched while this one's adjoint runs.
-template <int S>
+// 128 x 128, per 1024 positions: 172 us, where the block-wide walk with named
+// barriers took 250 and one position per block of this one 219.
+// kFull adds the projection sets and the kept far field: 4096 positions of a
+// difference map 765 us (one position per block: 1066, and 140 us more to add the
+// probe terms of all positions), 1024 positions with the far field kept 182 (233).
+template <int S, bool kFull>
 __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
   using W = WaveFft<S>;
   using P = WavePosition<S>;
@@ -685,6 +690,9 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
   constexpr int AP = S + 8;
   float* const amps = reinterpret_cast<float*>(smem4 + P::CELLS);
   const float invN = 1.0f / (float)N;
+  const bool ps = kFull && a.projection != 0;
+  const float px_ = 1.0f - a.pa - a.pb;  // projection x
+  const float py_ = 1.0f - a.pc;          // projection y
   const float2* __restrict__ spec = a.probe_spec;
   // `count` of the PARTS 16-byte pieces that each thread copies, from piece q on
   constexpr int PARTS = N / 4 / W::NT;
@@ -705,6 +713,7 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
   };
   int b = blockIdx.x;
   int row = a.amp_rows ? a.amp_rows[b] : b;
+  int prow = kFull && a.pos_rows ? a.pos_rows[b] : b;
   load_spectrum();
   const float2 at = P::position(a, a.positions, b);
   bool pos_ok = p.locate(a, at.x, at.y, 0);
@@ -723,6 +732,7 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
     const int next_row = a.amp_rows ? a.amp_rows[nb] : nb;
     const int next_prow = a.pos_rows ? a.pos_rows[nb] : nb;
     float2 next_at;
+    float2* const ew = ps ? a.exit_waves + (size_t)prow * N : nullptr;
     P cur = p;  // (patch corner of this position; p moves on to the next below)
     if (tid == 0) a.pos_round[b] = make_int2(p.x0, p.y0);
     // columns: spectrum x ramp, back to real space
@@ -761,6 +771,13 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
           for (int i = 0; i < 8; ++i) st_two(nobj + p.real(t, i), abs2(v[i]));
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = mul(v[i], o[i]);
+          if (ps) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const Cx2 wv = a.ew_valid ? from_pair(ld_cell(ew + p.real(t, i))) : v[i];
+              v[i] = fma_r(wv, py_, scale(v[i], a.pc));
+            }
+          }
           w.row_outer_store(t, v);
           tmem_wait_store();
         } else {
@@ -772,6 +789,13 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
           for (int i = 0; i < 8; ++i) {
             const int e = p.real(t, i);
             const Cx2 q = tmem_cell(pr, i);
+            if (ps) {
+              // new exit wave x w + a psi + b projected
+              const Cx2 psi = mul(q, o[i]);
+              const Cx2 wv = a.ew_valid ? from_pair(ld_cell(ew + e)) : psi;
+              v[i] = fma_r(v[i], a.pb, fma_r(psi, a.pa, scale(wv, px_)));
+              st_cell(ew + e, to_pair(v[i]));
+            }
             Cx2 g = conj_mul(q, v[i]);
             if (a.potential) {
               // Re(-i conj(O) conj(P) chi)
@@ -811,9 +835,14 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           A[i] = ld_two(amps + ((t >> 2) + W::RI * i) * AP + 8 * w.warp + 2 * (t & 3));
+        if (kFull && a.keep_farfield) {
+          float2* const far = a.scratch_f + (size_t)b * N;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) st_cell(far + p.fourier(t, i), to_pair(v[i]));
+        }
         if (a.det_mask) apply_mask(p, a.det_mask, t, v);
-        project(true, A, v, err2);
-        if (a.det_mask) apply_mask(p, a.det_mask, t, v);
+        project(!ps, A, v, err2);
+        if (a.det_mask && !ps) apply_mask(p, a.det_mask, t, v);
         w.col_outer_store(t, v);
       }
       __syncwarp();
@@ -832,6 +861,7 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
     load_spectrum();
     if (next < a.B) pos_ok = p.locate(a, next_at.x, next_at.y, k ^ 1);
     row = next_row;
+    prow = next_prow;
     __syncthreads();
     first = false;
     b = next;
@@ -856,23 +886,44 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
 // Position correction of a single-slice batch: the expressions of
 // position_correction_kernel. The shifted probe is transformed once per mode and
 // waits in st_probe (which the batch's reductions have consumed) for the second
-// direction.
-template <int S>
+// direction. For a single probe at 128 x 128 (kTmem) the blocks are resident and
+// the probe and the far field of the batch wait in tensor memory, the x derivative
+// in shared memory. Bound: L2 traffic, 580 KB a position (1090 through memory).
+// 128 x 128, 1024 positions: 197 us; through memory, with the sums of all threads
+// in double: 303; the block-wide walk: 465.
+template <int S, bool kTmem>
 __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchArgs a) {
   using W = WaveFft<S>;
   using P = WavePosition<S>;
   constexpr int N = W::N;
   extern __shared__ float4 smem4[];
-  __shared__ double red[5][W::NT / 32];
+  __shared__ double sums[5];
+  __shared__ uint32_t tmem_base;
+  constexpr int WORDS = 64 * W::TITER;  // tensor-memory columns of a warp
+  constexpr int COLS = WORDS * (W::WARPS / 4);
+  static_assert(!kTmem || (W::TASKS % 32 == 0 && W::WARPS % 4 == 0 && COLS <= 512),
+                "tensor memory");
 
-  const int b = blockIdx.x;
   const int tid = threadIdx.x;
-  const int M = a.M;
-  const int prow = a.pos_rows ? a.pos_rows[b] : b;
-  const int arow = a.amp_rows ? a.amp_rows[b] : b;
+  const int M = kTmem ? 1 : a.M;
   P p;
   p.carve(smem4);
   p.w.tables(tid);
+  uint32_t tm = 0;
+  if constexpr (kTmem) {
+    if (p.w.warp == 0) nn::tmem_alloc(&tmem_base, COLS);
+    nn::tc_fence_before();
+    __syncthreads();
+    nn::tc_fence_after();
+    tm = tmem_base + ((uint32_t)(p.w.warp & 3) << 21) + (p.w.warp >> 2) * WORDS;
+  }
+  // this thread's d|F|^2/dx samples, in its own slots
+  float2* const own_gx = reinterpret_cast<float2*>(smem4 + P::CELLS);
+
+#pragma unroll 1
+  for (int b = blockIdx.x; b < a.B; b += gridDim.x) {
+  const int prow = a.pos_rows ? a.pos_rows[b] : b;
+  const int arow = a.amp_rows ? a.amp_rows[b] : b;
   const float2 at = P::position(a, a.positions_rw, b);
   const bool pos_ok = p.locate(a, at.x, at.y, 0);
   const float posx = finite_or_zero(at.x);
@@ -921,8 +972,18 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             v[i] = scale(v[i], invN);
-            st_cell(stash + p.real(t, i), as_cell(v[i]));
+            if (!kTmem) st_cell(stash + p.real(t, i), as_cell(v[i]));
           }
+          if constexpr (kTmem) {
+            tmem_put(tm + 32 * it, v);
+            tmem_wait_store();
+          }
+        } else if constexpr (kTmem) {
+          uint32_t c[32];
+          tmem_get(tm + 32 * it, c);
+          tmem_wait_load(c);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = tmem_cell(c, i);
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) v[i] = as_cx2(ld_cell(stash + p.real(t, i)));
@@ -943,9 +1004,24 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
         const int t = w.lane + 32 * it;
         if (W::TASKS % 32 != 0 && t >= W::TASKS) break;
         Cx2 r[8], v[8];
+        const uint32_t tf = tm + 32 * (W::TITER + it);
+        if (!kTmem || dir == 0) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = from_pair(ld_cell(f0 + p.fourier(t, i)));
+          for (int i = 0; i < 8; ++i) r[i] = from_pair(ld_cell(f0 + p.fourier(t, i)));
+        }
         w.col_outer_load(t, v);
+        if constexpr (kTmem) {
+          if (dir == 0) {
+            tmem_put(tf, r);
+            tmem_wait_store();
+          } else {
+            uint32_t c[32];
+            tmem_get(tf, c);
+            tmem_wait_load(c);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) r[i] = tmem_cell(c, i);
+          }
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int e = p.fourier(t, i);
@@ -953,8 +1029,10 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
           float2 u = __fmul2_rn(dup(2.0f), add2(__fmul2_rn(d.re, r[i].re),
                                                 __fmul2_rn(d.im, r[i].im)));
           if (m > 0) u = add2(ld_two(g + e), u);
+          float2& kept = own_gx[(8 * it + i) * W::NT + tid];
           if (!last) {
-            st_two(g + e, u);
+            if (kTmem) kept = u;
+            else st_two(g + e, u);
             continue;
           }
           // the normal equations of this thread's samples
@@ -963,7 +1041,7 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
             est = add2(est, abs2(from_pair(ld_cell(
                                 a.scratch_f + ((size_t)b * M + k) * N + e))));
           const float2 A = __ldg(reinterpret_cast<const float2*>(amp + e));
-          const float2 gv = ld_two(gx + e);
+          const float2 gv = kTmem ? kept : ld_two(gx + e);
           auto add_terms = [&](float px, float py, float d2) {
             sxx = fmaf(px, px, sxx);
             sxy = fmaf(px, py, sxy);
@@ -978,9 +1056,32 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
       __syncthreads();  // the wave is rewritten by rows (dir 1) or the next mode
     }
   }
-  double s5[5] = {sxx, sxy, syy, sxd, syd};
-  block_sum5<W::NT>(s5, red);
-  if (tid == 0) correction_update(a, prow, posx, posy, pos_ok, s5);
+  // the block's sums, in double: a warp per sum over the threads' partials (the
+  // wave's shared memory is free by now)
+  float* const part = reinterpret_cast<float*>(smem4);
+  part[tid] = sxx;
+  part[W::NT + tid] = sxy;
+  part[2 * W::NT + tid] = syy;
+  part[3 * W::NT + tid] = sxd;
+  part[4 * W::NT + tid] = syd;
+  __syncthreads();
+  for (int k = w.warp; k < 5; k += W::WARPS) {
+    double x = 0.0;
+#pragma unroll
+    for (int j = 0; j < W::WARPS; ++j) x += part[k * W::NT + 32 * j + w.lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (w.lane == 0) sums[k] = x;
+  }
+  __syncthreads();
+  if (tid == 0) correction_update(a, prow, posx, posy, pos_ok, sums);
+  }
+  if constexpr (kTmem) {
+    nn::tc_fence_before();
+    __syncthreads();
+    nn::tc_fence_after();
+    if (p.w.warp == 0) nn::tmem_dealloc(tmem_base, COLS);
+  }
 }
 
 // |P_b|^2 of the sub-pixel shifted probe (mode 0), as probe_intensity_kernel: the
@@ -1059,11 +1160,13 @@ inline int resident_blocks(int B) {
   return B < sms ? B : sms;
 }
 
-// Blocks of the resident gradient-descent kernel for this batch (the rows of
-// st_probe that hold probe terms), 0 when the batch runs another kernel.
+// Blocks of the resident single-slice single-probe kernel for this batch (the rows
+// of st_probe that hold probe terms), 0 when the batch runs another kernel.
 template <int S>
 int wave_gd_blocks(const BatchArgs& a) {
-  return S == 128 && wave_plain(a) ? resident_blocks(a.B) : 0;
+  return S == 128 && !wave_mixed(a) && a.T == 1 && !a.forward_only && !a.exact_probe_grad
+             ? resident_blocks(a.B)
+             : 0;
 }
 
 template <int S>
@@ -1074,7 +1177,7 @@ cudaError_t launch_wave_position(const BatchArgs& a, cudaStream_t s) {
                                  : WavePosition<S>::smem_bytes(true);
   void (*fn)(BatchArgs) = wave_mixed(a) ? wave_position_kernel<S, 2> : wave_position_kernel<S, 1>;
   if constexpr (S == 128) {
-    if (blocks > 0) fn = wave_gd_kernel<S>;
+    if (blocks > 0) fn = wave_plain(a) ? wave_gd_kernel<S, false> : wave_gd_kernel<S, true>;
   } else {
     if (wave_plain(a)) fn = wave_position_kernel<S, 0>;
   }
@@ -1102,12 +1205,20 @@ cudaError_t launch_wave_intensity(const BatchArgs& a, cudaStream_t s) {
 template <int S>
 cudaError_t launch_wave_correction(const BatchArgs& a, cudaStream_t s) {
   using W = WaveFft<S>;
-  const size_t smem = WavePosition<S>::smem_bytes(false);
-  cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(wave_correction_kernel<S>),
-                                    (int)smem);
+  size_t smem = WavePosition<S>::smem_bytes(false);
+  void (*fn)(BatchArgs) = wave_correction_kernel<S, false>;
+  int blocks = a.B;
+  if constexpr (S == 128) {
+    if (a.M == 1 && resident_blocks(a.B) > 0) {
+      fn = wave_correction_kernel<S, true>;
+      smem = WavePosition<S>::smem_bytes(true);
+      blocks = resident_blocks(a.B);
+    }
+  }
+  cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(fn), (int)smem);
   if (e != cudaSuccess) return e;
   if ((e = launch_transmission(a, s)) != cudaSuccess) return e;
-  wave_correction_kernel<S><<<a.B, W::NT, smem, s>>>(a);
+  fn<<<blocks, W::NT, smem, s>>>(a);
   return cudaGetLastError();
 }
 
