@@ -371,90 +371,122 @@ __global__ void __launch_bounds__(kPreThreads) pattern_normalize_global_kernel(
 }
 
 // ------------------------------------------------------- perfect-tree kernels
-// Chain j (0..7) of a leaf of length l starting at element `lo`: r = a[lo + j],
-// then r += a[lo + j + 8 k] for k = 1 .. l/8 - 1 (values from `val`). Lane j of
-// an 8-lane group holds chain j; the group's lane 0 gets the leaf sum
-// ((r0 + r1) + (r2 + r3)) + ((r4 + r5) + (r6 + r7)) plus the l % 8 tail in order.
-template <typename Acc, typename V>
-__device__ __forceinline__ Acc leaf_chain_sum(const V& val, int lo, int l) {
+// Lane j (0..7) of an 8-lane group holds the sum of chain j of a leaf,
+// r = a[lo + j], then r += a[lo + j + 8 k] in order; the group's lane 0 gets
+// ((r0 + r1) + (r2 + r3)) + ((r4 + r5) + (r6 + r7)).
+template <typename Acc>
+__device__ __forceinline__ Acc combine_chains(Acc r) {
   const int j = threadIdx.x & 7;
-  const int groups = l >> 3;
-  Acc r = val(lo + j);
-  for (int k = 1; k < groups; ++k) r = acc_add(r, (Acc)val(lo + j + 8 * k));
   Acc o = __shfl_down_sync(0xffffffffu, r, 1, 8);
   if ((j & 1) == 0) r = acc_add(r, o);
   o = __shfl_down_sync(0xffffffffu, r, 2, 8);
   if ((j & 3) == 0) r = acc_add(r, o);
   o = __shfl_down_sync(0xffffffffu, r, 4, 8);
-  if (j == 0) {
-    r = acc_add(r, o);
-    for (int i = groups * 8; i < l; ++i) r = acc_add(r, (Acc)val(lo + i));
+  return j == 0 ? acc_add(r, o) : r;
+}
+
+// The pairwise sum of L = 2^levels <= 128 leaf sums by one warp: each lane adds
+// its L / 32 neighbours, then the lanes pair up (every sum is of two neighbouring
+// subtrees, so the order of the two does not matter). The total is in every lane.
+template <typename Acc>
+__device__ __forceinline__ Acc warp_tree(const Acc* vals, int L) {
+  const int lane = threadIdx.x & 31;
+  Acc r = 0;
+  if (L >= 128) {
+    const Acc* v = vals + 4 * lane;
+    r = acc_add(acc_add(v[0], v[1]), acc_add(v[2], v[3]));
+  } else if (L >= 64) {
+    r = acc_add(vals[2 * lane], vals[2 * lane + 1]);
+  } else if (lane < L) {
+    r = vals[lane];
   }
+  for (int s = 1; s < 32 && s < L; s <<= 1)
+    r = acc_add(r, __shfl_xor_sync(0xffffffffu, r, s));
   return r;
 }
 
-// In-place pairwise sum of q arrays of L = 2^levels leaf sums each (arrays at
-// vals + q * L): level by level, vals[j] += vals[j + s]; the totals land in
-// vals[q * L]. Called by all threads of the block.
-template <typename Acc>
-__device__ __forceinline__ void tree_add(Acc* vals, int q, int L) {
-  for (int s = 1; s < L; s <<= 1) {
-    const int pairs = L / (2 * s);
-    for (int t = threadIdx.x; t < q * pairs; t += blockDim.x) {
-      const int a = t / pairs, k = t - (t / pairs) * pairs;
-      Acc* v = vals + a * L + 2 * s * k;
-      v[0] = acc_add(v[0], v[s]);
-    }
-    __syncthreads();
-  }
-}
-
-// Centre of mass, perfect tree: block = 8 L threads (at least one warp), one
-// pattern per block, lane group g sums leaf g of the three quantities straight
-// from global memory (each warp load covers four 32-byte runs).
+// Centre of mass, perfect tree: block = 8 L threads (at least three warps), one
+// pattern per block, lane group g sums leaf g of the three quantities in one walk
+// straight from global memory (each warp load covers four 32-byte runs), and a
+// warp per quantity adds the leaves.
+// Bound: memory and the float additions' order (a chain's are serial). 4096
+// patterns of 128 x 128: 61 us; with a walk per quantity and two divisions an
+// element 168.
 template <int kMask>
-__global__ void __launch_bounds__(1024) pattern_com_kernel(
+__global__ void __launch_bounds__(1024, 2) pattern_com_kernel(
     const float* __restrict__ in, int Qx, int Qy, const void* __restrict__ mask, int leaf,
     int L, void* cx_out, void* cy_out) {
   using Px = MaskedPixel<kMask>;
   using Acc = typename Px::Acc;
   __shared__ Acc vals[3 * 128];
+  __shared__ Acc total[3];
   const int N = Qx * Qy;
-  const int g = threadIdx.x >> 3;
+  const int g = threadIdx.x >> 3, j = threadIdx.x & 7;
   const Px px{in + (size_t)blockIdx.x * N, mask};
-  // lanes past the last leaf (blocks of one warp) sum elements 0..7 and drop
+  // lanes past the last leaf (blocks of few leaves) sum elements 0..7 and drop
   // the result: every lane of a warp takes part in the shuffles
   const int lo = g < L ? g * leaf : 0;
-  const int len = g < L ? leaf : 8;
-  const Acc s0 = leaf_chain_sum<Acc>(px, lo, len);
-  const Acc s1 = leaf_chain_sum<Acc>(
-      [&](int e) { return acc_mul(px(e), (Acc)(e / Qy)); }, lo, len);
-  const Acc s2 = leaf_chain_sum<Acc>(
-      [&](int e) { return acc_mul(px(e), (Acc)(e - (e / Qy) * Qy)); }, lo, len);
-  if (g < L && (threadIdx.x & 7) == 0) {
+  const int groups = g < L ? leaf >> 3 : 1;
+  constexpr int kAhead = kMask == 0 ? 8 : 4;  // loads in flight
+  int x = (lo + j) / Qy, y = lo + j - x * Qy;
+  Acc s0 = 0, s1 = 0, s2 = 0;
+#pragma unroll 1
+  for (int k0 = 0; k0 < groups; k0 += kAhead) {
+    Acc v[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (k0 + u < groups) v[u] = px(lo + j + 8 * (k0 + u));
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (k0 + u >= groups) break;
+      const Acc vx = acc_mul(v[u], (Acc)x), vy = acc_mul(v[u], (Acc)y);
+      const bool first = u == 0 && k0 == 0;
+      s0 = first ? v[u] : acc_add(s0, v[u]);
+      s1 = first ? vx : acc_add(s1, vx);
+      s2 = first ? vy : acc_add(s2, vy);
+      for (y += 8; y >= Qy; y -= Qy) ++x;
+    }
+  }
+  s0 = combine_chains(s0);
+  s1 = combine_chains(s1);
+  s2 = combine_chains(s2);
+  if (g < L && j == 0) {
+    for (int t = lo + 8 * groups; t < lo + leaf; ++t) {  // the leaf's tail, in order
+      const Acc v = px(t);
+      s0 = acc_add(s0, v);
+      s1 = acc_add(s1, acc_mul(v, (Acc)(t / Qy)));
+      s2 = acc_add(s2, acc_mul(v, (Acc)(t - (t / Qy) * Qy)));
+    }
     vals[g] = s0;
     vals[L + g] = s1;
     vals[2 * L + g] = s2;
   }
   __syncthreads();
-  tree_add<Acc>(vals, 3, L);
+  const int w = threadIdx.x >> 5;
+  if (w < 3) {
+    const Acc t = acc_add((Acc)0, warp_tree(vals + w * L, L));
+    if ((threadIdx.x & 31) == 0) total[w] = t;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    const Acc t0 = acc_add((Acc)0, vals[0]);
-    static_cast<Acc*>(cx_out)[blockIdx.x] = acc_div(acc_add((Acc)0, vals[L]), t0);
-    static_cast<Acc*>(cy_out)[blockIdx.x] = acc_div(acc_add((Acc)0, vals[2 * L]), t0);
+    static_cast<Acc*>(cx_out)[blockIdx.x] = acc_div(total[1], total[0]);
+    static_cast<Acc*>(cy_out)[blockIdx.x] = acc_div(total[2], total[0]);
   }
 }
 
 // Normalisation, perfect tree: block = 8 L threads, one pattern per block. The
-// pattern is staged in shared memory, each thread forms its l/8 shifted values
-// (elements tid + k blockDim) in registers, writes them back in place, then the
-// lane groups sum the leaves and every thread writes its amplitudes.
-constexpr int kMaxPerThread = 16;  // l / 8 <= 128 / 8
-
-__global__ void __launch_bounds__(1024) pattern_normalize_kernel(
+// pattern is copied to shared memory (rows 8 samples apart from a multiple of 32,
+// so that the four rows a warp walks fall into different banks); each lane forms
+// the shifted values of its chain in order, adds them and writes their
+// amplitudes as it goes.
+// Bound: instruction issue (four taps, single roundings, the square root); two blocks
+// an SM, so that one copies while the other computes.
+// 4096 patterns of 128 x 128: 180 us; with the shifted pattern written back to
+// shared memory and one block an SM 314.
+__global__ void __launch_bounds__(1024, 2) pattern_normalize_kernel(
     const float* __restrict__ in, int Qx, int Qy, const int32_t* __restrict__ rows,
-    const float* __restrict__ cfx, const float* __restrict__ cfy, int crop_w, int leaf, int L,
-    float* __restrict__ amps, float* __restrict__ sums) {
+    const float* __restrict__ cfx, const float* __restrict__ cfy, int crop_w, int LD, int leaf,
+    int L, float* __restrict__ amps, float* __restrict__ sums) {
   extern __shared__ float4 smem4[];
   __shared__ float vals[128];
   float* pat = reinterpret_cast<float*>(smem4);
@@ -464,11 +496,27 @@ __global__ void __launch_bounds__(1024) pattern_normalize_kernel(
   const int o = blockIdx.x;
   const int r = rows ? rows[o] : o;
   const float* src = in + (size_t)r * N;
-  if ((N & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    const float4* s4 = reinterpret_cast<const float4*>(src);
-    for (int e = tid; e < N / 4; e += NT) smem4[e] = __ldg(s4 + e);
+  if ((Qy & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    const int q = Qy >> 2, di = NT / q, dj = NT - di * q;
+    int i = tid / q, c = tid - i * q;
+    for (int e = tid; e < N / 4; e += NT) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(pat + i * LD + 4 * c)),
+                   "l"(src + 4 * e)
+                   : "memory");
+      i += di;
+      c += dj;
+      if (c >= q) {
+        c -= q;
+        ++i;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
-    for (int e = tid; e < N; e += NT) pat[e] = __ldg(src + e);
+    for (int e = tid; e < N; e += NT) {
+      const int i = e / Qy;
+      pat[i * LD + e - i * Qy] = __ldg(src + e);
+    }
   }
 
   const float xs = -cfx[r], ys = -cfy[r];
@@ -478,67 +526,72 @@ __global__ void __launch_bounds__(1024) pattern_normalize_kernel(
   const float w00 = __fmul_rn(ux, uy), w10 = __fmul_rn(wx, uy);
   const float w01 = __fmul_rn(ux, wy), w11 = __fmul_rn(wx, wy);
   const int ixm = pmod((int)xf, Qx), iym = pmod((int)yf, Qy);
-  __syncthreads();
-
-  // shifted values of elements e = tid + k NT, (i, j) advanced incrementally
-  const int per = (N + NT - 1) / NT;
-  const int di = NT / Qy, dj = NT - (NT / Qy) * Qy;
-  float v[kMaxPerThread];
-  {
-    int i = tid / Qy, j = tid - (tid / Qy) * Qy;
-#pragma unroll
-    for (int k = 0; k < kMaxPerThread; ++k) {
-      if (k < per && tid + k * NT < N) {
-        int i0 = i - ixm;
-        if (i0 < 0) i0 += Qx;
-        int i1 = i0 - 1;
-        if (i1 < 0) i1 += Qx;
-        int j0 = j - iym;
-        if (j0 < 0) j0 += Qy;
-        int j1 = j0 - 1;
-        if (j1 < 0) j1 += Qy;
-        float t = __fmul_rn(pat[i0 * Qy + j0], w00);
-        t = __fadd_rn(t, __fmul_rn(pat[i1 * Qy + j0], w10));
-        t = __fadd_rn(t, __fmul_rn(pat[i0 * Qy + j1], w01));
-        t = __fadd_rn(t, __fmul_rn(pat[i1 * Qy + j1], w11));
-        v[k] = t;
-      }
-      i += di;
-      j += dj;
-      if (j >= Qy) {
-        j -= Qy;
-        ++i;
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kMaxPerThread; ++k)
-    if (k < per && tid + k * NT < N) pat[tid + k * NT] = v[k];
-  __syncthreads();
-
-  const int g = tid >> 3;
-  const float ls = leaf_chain_sum<float>([&](int e) { return pat[e]; }, g < L ? g * leaf : 0,
-                                  g < L ? leaf : 8);
-  if (g < L && (tid & 7) == 0) vals[g] = ls;
-
-  // amplitudes (numpy.maximum keeps its first argument unless it is below the second)
   const int Cx = crop_w > 0 ? 2 * crop_w : Qx;
   const int Cy = crop_w > 0 ? 2 * crop_w : Qy;
-  float* dst = amps + (size_t)o * Cx * Cy;
-  for (int e = tid; e < Cx * Cy; e += NT) {
-    int x = e / Cy, y = e - (e / Cy) * Cy;
-    if (crop_w > 0) {
-      if (x >= crop_w) x += Qx - Cx;
-      if (y >= crop_w) y += Qy - Cy;
+  float* const dst = amps + (size_t)o * Cx * Cy;
+  __syncthreads();
+
+  // the shifted values of row i: its two source rows, and where its samples go (a
+  // crop keeps the corners of crop_w samples a side)
+  const float *p0, *p1;
+  float* out;
+  bool kept;
+  auto set_row = [&](int i, bool write) {
+    int i0 = i - ixm;
+    if (i0 < 0) i0 += Qx;
+    int i1 = i0 - 1;
+    if (i1 < 0) i1 += Qx;
+    p0 = pat + i0 * LD;
+    p1 = pat + i1 * LD;
+    kept = write && (crop_w == 0 || i < crop_w || i >= Qx - crop_w);
+    out = dst + (crop_w > 0 && i >= crop_w ? i - (Qx - Cx) : i) * Cy;
+  };
+  // the value of column j; its amplitude goes out (numpy.maximum keeps its first
+  // argument unless it is below the second)
+  auto shifted = [&](int j) {
+    int j0 = j - iym;
+    if (j0 < 0) j0 += Qy;
+    int j1 = j0 - 1;
+    if (j1 < 0) j1 += Qy;
+    float t = __fmul_rn(p0[j0], w00);
+    t = __fadd_rn(t, __fmul_rn(p1[j0], w10));
+    t = __fadd_rn(t, __fmul_rn(p0[j1], w01));
+    t = __fadd_rn(t, __fmul_rn(p1[j1], w11));
+    const bool column = crop_w == 0 || j < crop_w || j >= Qy - crop_w;
+    const int jo = crop_w > 0 && j >= crop_w ? j - (Qy - Cy) : j;
+    if (kept && column) out[jo] = __fsqrt_rn(!(t >= 0.0f) && !isnan(t) ? 0.0f : t);
+    return t;
+  };
+  const int g = tid >> 3, c = tid & 7;
+  const bool in_leaf = g < L;
+  const int lo = in_leaf ? g * leaf : 0;
+  const int groups = in_leaf ? leaf >> 3 : 1;
+  int i = (lo + c) / Qy, j = lo + c - i * Qy;
+  float ls = 0.0f;
+  for (int k = 0; k < groups;) {
+    set_row(i, in_leaf);
+    const int n = min(groups - k, (Qy - 1 - j) / 8 + 1);  // steps within the row
+    if (k == 0) {  // (the chain starts with its first value, not with 0 + it)
+      ls = shifted(j);
     }
-    float a = pat[x * Qy + y];
-    if (!(a >= 0.0f) && !isnan(a)) a = 0.0f;
-    dst[e] = __fsqrt_rn(a);
+#pragma unroll 4
+    for (int u = k == 0 ? 1 : 0; u < n; ++u) ls = acc_add(ls, shifted(j + 8 * u));
+    k += n;
+    for (j += 8 * n; j >= Qy; j -= Qy) ++i;
+  }
+  ls = combine_chains(ls);
+  if (in_leaf && c == 0) {
+    for (int e = lo + 8 * groups; e < lo + leaf; ++e) {
+      set_row(e / Qy, true);
+      ls = acc_add(ls, shifted(e - (e / Qy) * Qy));
+    }
+    vals[g] = ls;
   }
   __syncthreads();
-  tree_add<float>(vals, 1, L);
-  if (tid == 0) sums[o] = __fadd_rn(0.0f, vals[0]);
+  if (tid < 32) {
+    const float t = warp_tree(vals, L);
+    if (tid == 0) sums[o] = __fadd_rn(0.0f, t);
+  }
 }
 
 // Number of leaves of the pairwise tree over n values (host side, for sizing).
@@ -579,7 +632,7 @@ cudaError_t launch_pattern_com_t(const float* in, int num, int Qx, int Qy, const
   int leaf = 0, levels = 0;
   if (pairwise_perfect(N, leaf, levels)) {
     const int L = 1 << levels;
-    const int threads = 8 * L < 32 ? 32 : 8 * L;
+    const int threads = 8 * L < 96 ? 96 : 8 * L;  // (a warp for each of the three sums)
     pattern_com_kernel<kMask><<<num, threads, 0, s>>>(in, Qx, Qy, mask, leaf, L, cx, cy);
     return cudaGetLastError();
   }
@@ -634,11 +687,12 @@ cudaError_t launch_pattern_normalize(const float* in, int Qx, int Qy, const int3
   if (pairwise_perfect(N, leaf, levels)) {
     const int L = 1 << levels;
     const int threads = 8 * L < 32 ? 32 : 8 * L;
-    const size_t smem = sizeof(float) * (size_t)N;
+    const int LD = Qy >= 32 ? Qy + 8 : Qy;  // (short rows: at most 64 KB as they are)
+    const size_t smem = sizeof(float) * (size_t)Qx * LD;
     cudaError_t e = set_smem((const void*)pattern_normalize_kernel, smem);
     if (e != cudaSuccess) return e;
     pattern_normalize_kernel<<<num_out, threads, smem, s>>>(in, Qx, Qy, rows, cfx, cfy, crop_w,
-                                                            leaf, L, amps, sums);
+                                                            LD, leaf, L, amps, sums);
     return cudaGetLastError();
   }
   const int L = pairwise_leaf_count(N);
