@@ -406,14 +406,17 @@ __global__ void __launch_bounds__(kEwThreads) staged_resample_back_kernel(BatchA
 
 // err[b] = the position's chunk partials summed in order; NaN for a non-finite
 // position (reported as PTYCHO_ERR_NONFINITE).
-__global__ void staged_error_kernel(BatchArgs a, int chunks) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.B) return;
+__device__ __forceinline__ void position_error(const BatchArgs& a, int b, int chunks) {
   float t = 0.0f;
   for (int c = 0; c < chunks; ++c) t += a.err_part[(size_t)b * chunks + c];
   const int prow = a.pos_rows ? a.pos_rows[b] : b;
   const bool ok = isfinite(a.positions[2 * prow]) && isfinite(a.positions[2 * prow + 1]);
   a.err[b] = ok ? t : __int_as_float(0x7fc00000);
+}
+
+__global__ void staged_error_kernel(BatchArgs a, int chunks) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < a.B) position_error(a, b, chunks);
 }
 
 // Adjoint at slice s: chi_m = W_m / N; object terms summed over the modes in
@@ -450,6 +453,280 @@ __global__ void __launch_bounds__(kEwThreads) staged_adjoint_kernel(BatchArgs a,
     a.st_nobj[((size_t)s * a.B + b) * N + e] = pn;
     if (s == 0 && !a.nprobe_from_object) a.st_nprobe[(size_t)b * N + e] = c_abs2(o);
   }
+}
+
+// ------------------------------------------- fused passes, 256 x 256 detectors
+// Without resampling, the passes at 256 x 256 are fused into strips of 16 lines
+// that stay in registers: 256 threads, 16 samples each, lane (l, q) holding
+// samples q + 16 k of line l before and after a transform. Columns: spectrum and
+// ramps -> inverse; forward -> projection or propagator -> inverse. Rows: inverse
+// -> overlap -> forward; inverse -> adjoint (-> forward). A transform is two
+// radix-16 passes with one exchange through shared memory (the passes and
+// twiddles of Schedule<256>, so the same bits).
+// Bound: memory latency and traffic; a single-slice position crosses memory 4 times
+// (6.6 MB) instead of 10 (13 MB). 128 positions, one slice: 20 + 50 + 51 + 65 us
+// where the separate passes took 400. Smaller groups of positions that stay in L2
+// through the four passes were slower (16, 32, 64 at a time: 2.81, 2.47, 2.20 ms a
+// pass of 1024 against 2.22 whole).
+constexpr int kFusedSize = 256;
+constexpr int kFusedLine = 16 * 17 + 1;  // pitch of a line in the exchange buffer
+
+template <bool ROWS>
+struct Strip {
+  int q, l, l0;
+  float2* line;
+  const float2* tw;
+  // strip `k` of a wave: its lines start at 16 k
+  __device__ __forceinline__ Strip(int k, float2* buf, float2* table) {
+    const int tid = threadIdx.x;
+    q = ROWS ? tid & 15 : tid >> 4;
+    l = ROWS ? tid >> 4 : tid & 15;
+    l0 = kLines * k;
+    line = buf + l * kFusedLine;
+    tw = table;
+    fill_twiddles<kFusedSize, kLineThreads>(table);
+    __syncthreads();
+  }
+  __device__ __forceinline__ int x(int k) const { return ROWS ? l0 + l : q + 16 * k; }
+  __device__ __forceinline__ int y(int k) const { return ROWS ? q + 16 * k : l0 + l; }
+  __device__ __forceinline__ int at(int k) const { return x(k) * kFusedSize + y(k); }
+  __device__ __forceinline__ void load(const float2* w, float2 (&v)[16]) const {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = w[at(k)];
+  }
+  __device__ __forceinline__ void store(float2* w, const float2 (&v)[16]) const {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) w[at(k)] = v[k];
+  }
+  template <int DIR>
+  __device__ __forceinline__ void transform(float2 (&v)[16]) const {
+    dft<16, DIR>(v);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) line[17 * q + k] = v[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = line[17 * k + q];
+#pragma unroll
+    for (int k = 1; k < 16; ++k) {
+      float2 t = tw[q * k];
+      if (DIR > 0) t.y = -t.y;
+      v[k] = c_mul(v[k], t);
+    }
+    dft<16, DIR>(v);
+    __syncthreads();  // the buffer is free for the next transform
+  }
+};
+
+enum FusedColumns { kShift, kProject, kPropagate };
+
+// blockIdx.x = 16 wave + strip; kShift: W = IFFT(spec ramps) along x, kProject
+// (one probe): W = IFFT(G(FFT(W))), kPropagate: W = IFFT(h FFT(W))
+template <int kKind>
+__global__ void __launch_bounds__(kLineThreads, 3)
+    fused_columns_kernel(BatchArgs a, const float2* __restrict__ ramps, float2* W,
+                         const float2* __restrict__ h, int conjugate) {
+  constexpr int N = kFusedSize * kFusedSize;
+  __shared__ float2 buf[kLines * kFusedLine];
+  __shared__ float2 table[kFusedSize];
+  const int wave = blockIdx.x >> 4, strip = blockIdx.x & 15;
+  const Strip<false> p(strip, buf, table);
+  float2* const w = W + (size_t)wave * N;
+  float2 v[16];
+  if constexpr (kKind == kShift) {
+    const int b = wave / a.M, m = wave % a.M;
+    const float2* rx = ramps + (size_t)b * 2 * kFusedSize;
+    const float2 ry = rx[kFusedSize + p.y(0)];
+    const float2* spec = a.probe_spec + (size_t)m * N;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = __ldg(spec + p.at(k));
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = c_mul(v[k], c_mul(rx[p.x(k)], ry));
+  } else {
+    p.load(w, v);
+    if constexpr (kKind == kProject) {
+      const int arow = a.amp_rows ? a.amp_rows[wave] : wave;
+      const float* amp = a.amplitudes + (size_t)arow * N;
+      float A[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) A[k] = __ldg(amp + p.at(k));
+      p.template transform<-1>(v);
+      const bool masked = a.det_mask != nullptr;
+      float err = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const float mk = masked ? a.det_mask[p.at(k)] : 1.0f;
+        err += project_pixel<true>(a, &v[k], A[k], mk, masked);
+      }
+      __shared__ float red[kLineThreads / 32];
+      const float t = block_sum<kLineThreads>(err, red);
+      if (threadIdx.x == 0) a.err_part[blockIdx.x] = t;
+      if (a.forward_only) return;
+    } else {
+      p.template transform<-1>(v);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        float2 hv = __ldg(h + p.at(k));
+        if (conjugate) hv.y = -hv.y;
+        v[k] = c_mul(v[k], hv);
+      }
+    }
+  }
+  p.template transform<+1>(v);
+  p.store(w, v);
+}
+
+// blockIdx.x = 16 position + strip, rows of every mode. Forward (kAdjoint false):
+// W_m = FFT(P_{s,m} O_s) with P_{s,m} = IFFT(W_m) / N stashed. Adjoint: the terms
+// of staged_adjoint_kernel, and W_m = FFT(chi_m conj(O_s)) for s > 0. kModes: the
+// object terms of M > 1 modes are summed in registers.
+// The patch and P travel to the thread's own slots of shared memory while the
+// first transform runs. chunks > 0: also the error of the position from its
+// partials.
+constexpr int kSlots = 16 * kLineThreads;
+constexpr int kRowsSmem = (int)sizeof(float2) * (kLines * kFusedLine + kFusedSize);
+
+template <bool kAdjoint, bool kModes>
+__global__ void __launch_bounds__(kLineThreads, 2)
+    fused_rows_kernel(BatchArgs a, float2* W, int s, int chunks) {
+  constexpr int N = kFusedSize * kFusedSize;
+  extern __shared__ float2 fused_smem[];
+  float2* const buf = fused_smem;
+  float2* const table = buf + kLines * kFusedLine;
+  float2* const own_o = table + kFusedSize + threadIdx.x;  // 16 slots, kLineThreads apart
+  float2* const own_p = own_o + kSlots;                    // (adjoint)
+  const int b = blockIdx.x >> 4, strip = blockIdx.x & 15;
+  const Strip<true> p(strip, buf, table);
+  if (kAdjoint && chunks > 0 && strip == 0 && threadIdx.x == 0) position_error(a, b, chunks);
+  const int2 r = a.pos_round[b];
+  const float invN = 1.0f / (float)N;
+  int ox = pmod(r.x - kFusedSize / 2, a.Px) + (p.x(0) + kFusedSize / 2) % kFusedSize;
+  if (ox >= a.Px) ox -= a.Px;
+  const int by = pmod(r.y - kFusedSize / 2, a.Py);
+  const size_t row = ((size_t)s * a.Px + ox) * a.Py;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    int oy = by + (p.y(k) + kFusedSize / 2) % kFusedSize;
+    if (oy >= a.Py) oy -= a.Py;
+    if (a.potential) {
+      own_o[k * kLineThreads].x = reinterpret_cast<const float*>(a.object)[row + oy];
+    } else {
+      copy_async8(own_o + k * kLineThreads, reinterpret_cast<const float2*>(a.object) + row + oy);
+    }
+  }
+  if (a.potential) {
+#pragma unroll 1
+    for (int k = 0; k < 16; ++k) {  // (rolled: the slow path of sincosf is long)
+      float2& o = own_o[k * kLineThreads];
+      float sv, cv;
+      sincosf(o.x, &sv, &cv);
+      o = make_float2(cv, sv);
+    }
+  }
+  float2 g[16];
+  float pn[16];
+  float2* const go = a.st_obj + ((size_t)s * a.B + b) * N;
+  float* const no = a.st_nobj + ((size_t)s * a.B + b) * N;
+  const int M = kModes ? a.M : 1;
+#pragma unroll 1
+  for (int m = 0; m < M; ++m) {
+    float2* const w = W + ((size_t)b * M + m) * N;
+    float2* const st = stash(a, s, b, m);
+    float2 v[16];
+    p.load(w, v);
+    if constexpr (kAdjoint) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) copy_async8(own_p + k * kLineThreads, st + p.at(k));
+    }
+    p.template transform<+1>(v);
+    copy_async_wait();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = c_scale(v[k], invN);
+    if constexpr (!kAdjoint) {
+      p.store(st, v);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = c_mul(v[k], own_o[k * kLineThreads]);
+      p.template transform<-1>(v);
+      p.store(w, v);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const float2 pv = own_p[k * kLineThreads], o = own_o[k * kLineThreads];
+        const float2 gm = object_term(a.potential, o, pv, v[k]);
+        if (!kModes) {
+          go[p.at(k)] = gm;
+          no[p.at(k)] = c_abs2(pv);
+        } else {
+          g[k] = m == 0 ? gm : c_add(g[k], gm);
+          pn[k] = m == 0 ? c_abs2(pv) : pn[k] + c_abs2(pv);
+        }
+        v[k] = c_conj_mul(o, v[k]);
+      }
+      if (s > 0) {
+        p.template transform<-1>(v);
+        p.store(w, v);
+      } else {
+        p.store(a.st_probe + ((size_t)b * M + m) * N, v);
+      }
+    }
+  }
+  if constexpr (kAdjoint) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      if (kModes) {
+        go[p.at(k)] = g[k];
+        no[p.at(k)] = pn[k];
+      }
+      if (s == 0 && !a.nprobe_from_object) 
+        a.st_nprobe[(size_t)b * N + p.at(k)] = c_abs2(own_o[k * kLineThreads]);
+    }
+  }
+}
+
+cudaError_t launch_fused_positions(const BatchArgs& a, cudaStream_t s) {
+  constexpr int N = kFusedSize * kFusedSize;
+  const int BM = a.B * a.M;
+  float2* ramps = reinterpret_cast<float2*>(a.st_nobj);
+  float2* W = a.scratch_f;
+  const bool single = a.M == 1 && !a.mixed_formula;
+  const auto rows_forward = a.M > 1 ? fused_rows_kernel<false, true> : fused_rows_kernel<false, false>;
+  const auto rows_adjoint = a.M > 1 ? fused_rows_kernel<true, true> : fused_rows_kernel<true, false>;
+  const int forward_smem = kRowsSmem + (int)sizeof(float2) * kSlots;
+  const int adjoint_smem = forward_smem + (int)sizeof(float2) * kSlots;
+  cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(rows_forward), forward_smem);
+  if (e != cudaSuccess) return e;
+  e = ensure_smem_limit(reinterpret_cast<const void*>(rows_adjoint), adjoint_smem);
+  if (e != cudaSuccess) return e;
+  staged_ramps_kernel<<<a.B, 256, 0, s>>>(a, ramps, 0);
+  fused_columns_kernel<kShift><<<16 * BM, kLineThreads, 0, s>>>(a, ramps, W, nullptr, 0);
+  for (int sl = 0; sl < a.T; ++sl) {
+    rows_forward<<<16 * a.B, kLineThreads, forward_smem, s>>>(a, W, sl, 0);
+    if (sl + 1 < a.T)
+      fused_columns_kernel<kPropagate><<<16 * BM, kLineThreads, 0, s>>>(
+          a, nullptr, W, a.props + (size_t)sl * N, 0);
+  }
+  int chunks = 16;
+  if (single) {
+    fused_columns_kernel<kProject><<<16 * BM, kLineThreads, 0, s>>>(a, nullptr, W, nullptr, 0);
+  } else {
+    chunks = chunks_of(N);
+    if ((e = lines<-1, false>(W, W, BM, 256, 256, 256, 1.0f, nullptr, s)) != cudaSuccess) return e;
+    staged_projection_kernel<false><<<dim3(a.B, chunks), kEwThreads, 0, s>>>(a, W);
+    if (!a.forward_only &&
+        (e = lines<+1, false>(W, W, BM, 256, 256, 256, 1.0f, nullptr, s)) != cudaSuccess)
+      return e;
+  }
+  if (a.forward_only) {
+    staged_error_kernel<<<(a.B + 255) / 256, 256, 0, s>>>(a, chunks);
+    return cudaGetLastError();
+  }
+  for (int sl = a.T - 1; sl >= 0; --sl) {
+    rows_adjoint<<<16 * a.B, kLineThreads, adjoint_smem, s>>>(a, W, sl,
+                                                                sl + 1 == a.T ? chunks : 0);
+    if (sl > 0)
+      fused_columns_kernel<kPropagate><<<16 * BM, kLineThreads, 0, s>>>(
+          a, nullptr, W, a.props + (size_t)(sl - 1) * N, 1);
+  }
+  return cudaGetLastError();
 }
 
 // |P_b|^2 = |W / N|^2, abs() then square as numpy forms it
@@ -596,6 +873,7 @@ cudaError_t launch_staged_spectrum(const BatchArgs& a, cudaStream_t s) {
 
 cudaError_t launch_staged_positions(const BatchArgs& a, cudaStream_t s) {
   if (!staged_batch_supported(a)) return cudaErrorNotSupported;
+  if (!a.resample && a.Sx == kFusedSize && a.Sy == kFusedSize) return launch_fused_positions(a, s);
   const int N = a.Sx * a.Sy;
   const int BM = a.B * a.M;
   float2* ramps = reinterpret_cast<float2*>(a.st_nobj);

@@ -178,7 +178,7 @@ __device__ __forceinline__ float rsqrt_approx(float v) {
   return r;
 }
 // asynchronous 8-byte copy from global to shared memory
-__device__ __forceinline__ void copy_async8(float2* dst, const float* src) {
+__device__ __forceinline__ void copy_async8(float2* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
                    (unsigned)__cvta_generic_to_shared(dst)),
                "l"(src)
