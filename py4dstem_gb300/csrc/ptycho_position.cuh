@@ -96,8 +96,9 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // mixed-state multislice; modes 1-3 are gradient descent with no projection
 // sets, forward-only pass, kept far fields or exact probe gradient; mode 4 runs
 // every variant of the mixed-state multislice model (its far fields always stay
-// in scratch_f).
-template <int SX, int SY, int NT, int kMode>
+// in scratch_f). ENT < NT (mode 1): the error is summed in the order of a block of
+// ENT threads.
+template <int SX, int SY, int NT, int kMode, int ENT>
 __device__ __forceinline__ void position_one(const BatchArgs& a, const int b, float* red) {
   constexpr bool kPlain = kMode >= 1 && kMode <= 3;
   constexpr bool kT1 = kMode == 1 || kMode == 2;
@@ -111,7 +112,7 @@ __device__ __forceinline__ void position_one(const BatchArgs& a, const int b, fl
   float2* twy = twx + SX;
   float2* rpx = twy + SY;
   float2* rpy = rpx + SX;
-  float* itot = reinterpret_cast<float*>(rpy + SY);  // N floats, mixed only
+  float* itot = reinterpret_cast<float*>(rpy + SY);  // N floats, mixed or ENT < NT only
 
   const int tid = threadIdx.x;
   const int T = kT1 ? 1 : a.T;
@@ -422,7 +423,11 @@ __device__ __forceinline__ void position_one(const BatchArgs& a, const int b, fl
         const float af = c_abs(f);
         const float A = av[i];
         const float d = A - af;
-        err += d * d;
+        if constexpr (ENT == NT) {
+          err += d * d;
+        } else {
+          itot[e] = d;
+        }
         // A exp(i angle F) (- F for gradient descent), one division per pixel
         const float q = af > 0.0f ? A / af : 0.0f;
         float2 r = af > 0.0f ? c_scale(f, q) : make_float2(A, 0.0f);
@@ -435,6 +440,14 @@ __device__ __forceinline__ void position_one(const BatchArgs& a, const int b, fl
       }
       if (!fwd) {
         __syncthreads();
+        if constexpr (ENT < NT) {
+          if (tid < ENT) {
+            for (int i = 0; i < N / ENT; ++i) {
+              const float d = itot[tid + i * ENT];
+              err += d * d;
+            }
+          }
+        }
         fft2d<SX, SY, NT, +1>(buf, twx, twy);
       }
     } else {
@@ -659,10 +672,10 @@ done:
 
 // One block per position. (A persistent form, one block per SM walking the
 // batch, measured 2% slower at 128 x 128 and was dropped.)
-template <int SX, int SY, int NT, int kMode>
+template <int SX, int SY, int NT, int kMode, int ENT = NT>
 __global__ void __launch_bounds__(NT, 1) position_kernel(BatchArgs a) {
   __shared__ float red[NT / 32];
-  position_one<SX, SY, NT, kMode>(a, blockIdx.x, red);
+  position_one<SX, SY, NT, kMode, ENT>(a, blockIdx.x, red);
 }
 
 // Position correction of one batch (ptychographic_methods.py:2071-2225), run
@@ -1111,6 +1124,19 @@ cudaError_t launch_position_t(const BatchArgs& a, cudaStream_t s) {
                    : a.T == 1 ? (a.M == 1 && !a.mixed_formula ? 1 : 2)
                    : 3;
   timing_before(s);
+  if constexpr (SX * SY <= 64 * 64) {
+    // a small batch leaves most of an SM to each position: twice the threads
+    if (small_batch(a)) {
+      const size_t wide = Layout<SX, SY>::smem_bytes(true);
+      const cudaError_t e0 = ensure_smem_limit(
+          reinterpret_cast<const void*>(position_kernel<SX, SY, 2 * NT, 1, NT>), (int)wide);
+      if (e0 != cudaSuccess) return e0;
+      position_kernel<SX, SY, 2 * NT, 1, NT><<<a.B, 2 * NT, wide, s>>>(a);
+      const cudaError_t e = cudaGetLastError();
+      timing_after(s);
+      return e;
+    }
+  }
   switch (mode) {
     case 1: position_kernel<SX, SY, NT, 1><<<a.B, NT, smem, s>>>(a); break;
     case 2: position_kernel<SX, SY, NT, 2><<<a.B, NT, smem, s>>>(a); break;

@@ -93,8 +93,8 @@ __device__ __forceinline__ void mark_nonfinite(const BatchArgs& a, float2 v) {
 constexpr int kRowsPerLane = 8;  // tile rows one lane visits per list entry (every other row)
 
 // A cluster of C blocks (8 warps each) per 16x16 object tile and slice; warp w of
-// block r takes part 8 r + w of the batch or, for small batches (in_turn, C = 1),
-// every eighth of the positions that touch the tile. Its lanes test 32 positions at a time
+// block r takes part 8 r + w of the batch or, for small batches (kInTurn, C = 1),
+// every eighth of the positions that touch the tile, four at a time. Its lanes test 32 positions at a time
 // for a patch that touches the tile (with the tile origin in patch coordinates)
 // and the warp then visits the hits in order. For a hit, lane l covers tile column
 // l % 16 of rows l / 16, l / 16 + 2, ..., so each warp load reads two whole
@@ -107,7 +107,8 @@ constexpr int kRowsPerLane = 8;  // tile rows one lane visits per list entry (ev
 // Bound: HBM and load latency (each warp keeps 16 loads in flight): 58 us per 1024
 // positions at 128 x 128 on a 319 x 319 object (3.5 TB/s), where a block-wide
 // list of the tile's positions took 99 us, with 8 warps waiting for the list's
-// barriers and one block a tile (up to 600 positions) running on alone.
+// barriers and one block a tile (up to 600 positions) running on alone. 64 x 64,
+// batch 64: 8.4 us with four positions at a time, 13.1 with one.
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -136,8 +137,9 @@ __device__ __forceinline__ float2 cluster_load2(const float2* p, uint32_t rank) 
   return v;
 }
 
-__global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C,
-                                                             int in_turn) {
+template <bool kInTurn>
+__global__ void __launch_bounds__(NT, kInTurn ? 1 : 4) object_reduce_kernel(BatchArgs a, int C) {
+  constexpr int kHits = kInTurn ? 4 : 1;  // positions whose terms are loaded at once
   __shared__ float part[NT / 32][3][NT];  // per-warp partials (g.x, g.y, n) per tile pixel
   __shared__ float red[NT / 32];
   static_assert(kTile * kTile == NT && kTile == 2 * kRowsPerLane, "tile layout");
@@ -162,8 +164,8 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C
   const int lane = tid & 31, warp = tid >> 5;
   const int parts = C * (NT / 32);
   const int per = (a.B + parts - 1) / parts;
-  const int b0 = in_turn ? 0 : min(a.B, (rank * (NT / 32) + warp) * per);
-  const int b1 = in_turn ? a.B : min(a.B, b0 + per);
+  const int b0 = kInTurn ? 0 : min(a.B, (rank * (NT / 32) + warp) * per);
+  const int b1 = kInTurn ? a.B : min(a.B, b0 + per);
   int turn = 0;  // the next hit's place among the tile's
 
   // staging axes: u is the slow one (rows), v the contiguous one
@@ -194,12 +196,19 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C
       d = (dx << 16) | dy;
     }
     unsigned hits = __ballot_sync(0xffffffffu, hit);
-    if (in_turn) {
+    if (kInTurn) {
       const int place = turn + __popc(hits & ((1u << lane) - 1u));
       turn += __popc(hits);
       hits = __ballot_sync(0xffffffffu, hit && place % (NT / 32) == warp);
     }
     while (hits) {
+      float2 v[kHits][kRowsPerLane];
+      float w[kHits][kRowsPerLane];
+      bool any[kHits];
+#pragma unroll
+      for (int h = 0; h < kHits; ++h) {
+      any[h] = hits != 0;
+      if (!any[h]) break;
       const int bit = __ffs(hits) - 1;
       hits &= hits - 1;
       const int du0 = __shfl_sync(0xffffffffu, d, bit);
@@ -211,27 +220,30 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C
       const bool vok = iv < tv && sv < Sv;
       const int lv = sv >= hv ? sv - hv : sv + hv;
       const size_t col = (size_t)(base + bit) * N + lv;
-      float2 v[kRowsPerLane];
-      float w[kRowsPerLane];
 #pragma unroll
       for (int k = 0; k < kRowsPerLane; ++k) {
         const int iu = iu0 + 2 * k;
         int su = du + iu;
         if (su >= Pu) su -= Pu;
-        v[k] = make_float2(0.f, 0.f);
-        w[k] = 0.f;
+        v[h][k] = make_float2(0.f, 0.f);
+        w[h][k] = 0.f;
         if (vok && iu < tu && su < Su) {
           const int lu = su >= hu ? su - hu : su + hu;
           const size_t e = col + (size_t)lu * Sv;
-          if (!a.nobj_only) v[k] = st[e];
-          w[k] = sn[e];
+          if (!a.nobj_only) v[h][k] = st[e];
+          w[h][k] = sn[e];
         }
       }
+      }
 #pragma unroll
-      for (int k = 0; k < kRowsPerLane; ++k) {
-        gx[k] += v[k].x;
-        gy[k] += v[k].y;
-        gn[k] += w[k];
+      for (int h = 0; h < kHits; ++h) {
+        if (!any[h]) break;
+#pragma unroll
+        for (int k = 0; k < kRowsPerLane; ++k) {
+          gx[k] += v[h][k].x;
+          gy[k] += v[h][k].y;
+          gn[k] += w[h][k];
+        }
       }
     }
   }
@@ -291,7 +303,7 @@ __global__ void __launch_bounds__(NT, 4) object_reduce_kernel(BatchArgs a, int C
 cudaError_t launch_object_reduce(const BatchArgs& a, int ntiles, cudaStream_t s) {
   const bool small = small_batch(a);
   const int C = ntiles * a.T <= 600 && a.B >= 128 && !small ? 2 : 1;
-  const int in_turn = small;
+  auto fn = small ? object_reduce_kernel<true> : object_reduce_kernel<false>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ntiles * C, a.T);
   cfg.blockDim = dim3(NT);
@@ -303,7 +315,7 @@ cudaError_t launch_object_reduce(const BatchArgs& a, int ntiles, cudaStream_t s)
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = C > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, object_reduce_kernel, a, C, in_turn);
+  return cudaLaunchKernelEx(&cfg, fn, a, C);
 }
 
 __global__ void __launch_bounds__(NT) object_update_kernel(BatchArgs a, int ntiles) {
@@ -638,7 +650,9 @@ cudaError_t launch_probe_finish_t(const BatchArgs& a, cudaStream_t s) {
 
 // The probe side after probe_reduce_kernel: the sums, the update and, with
 // prepare_spectrum, the next batch's spectrum. Probes that are not square (and
-// the transposed staging of the register-resident kernel) take one kernel a step.
+// the transposed staging of the register-resident kernel) take one kernel a step,
+// and so do 256 x 256 ones: eight blocks need 54 us for their sums, the four
+// kernels 30.
 cudaError_t launch_probe_finish(const BatchArgs& a, cudaStream_t s) {
   if (a.Sx == a.Sy && !a.staging_t) {
     switch (a.Sx) {
@@ -647,7 +661,6 @@ cudaError_t launch_probe_finish(const BatchArgs& a, cudaStream_t s) {
       case 64: return launch_probe_finish_t<64>(a, s);
       case 96: return launch_probe_finish_t<96>(a, s);
       case 128: return launch_probe_finish_t<128>(a, s);
-      case 256: return launch_probe_finish_t<256>(a, s);
       default: break;
     }
   }
@@ -907,20 +920,24 @@ __global__ void __launch_bounds__(NT) probe_mix_kernel(int M, int N, const float
 }
 
 // Eigen-decomposition of the M x M Hermitian Gram matrix on the device (cyclic
-// Jacobi in double, one thread; M <= 16), then the mixing coefficients of the
+// Jacobi in double, one warp; M <= 16), then the mixing coefficients of the
 // orthogonalised modes: mode i = sum_j coeffs[i*M+j] P_j with the eigenvectors
 // ordered by decreasing eigenvalue (= decreasing mode intensity), each
 // eigenvector's phase fixed so that its largest component is real and positive.
 // Rotation of pair (p, q): remove the phase of g_pq, then the real Jacobi
 // rotation t = sgn(tau)/(|tau| + sqrt(1 + tau^2)), tau = (g_qq - g_pp)/(2|g_pq|).
-// At most 32 sweeps; each sweep visits every pair once.
-__global__ void probe_eigh_kernel(int M, const float2* gram, float2* coeffs) {
+// At most 32 sweeps; each sweep visits every pair once. Every lane forms the
+// rotation, lane k < M turns row and column k.
+// Bound: the latency of float64 in the chain of rotations. Four modes: 104 us, one
+// thread 206.
+__global__ void __launch_bounds__(32) probe_eigh_kernel(int M, const float2* gram, float2* coeffs) {
   __shared__ double2 A[16][16];
   __shared__ double2 V[16][16];
   __shared__ double w[16];
   __shared__ int order[16];
-  if (threadIdx.x != 0) return;
-  for (int i = 0; i < M; ++i)
+  const int k = threadIdx.x;
+  if (k < M) {
+    const int i = k;
     for (int j = 0; j < M; ++j) {
       // upper triangle is the reference's input (eigh with UPLO='U')
       const float2 g = i <= j ? gram[i * M + j] : gram[j * M + i];
@@ -928,6 +945,8 @@ __global__ void probe_eigh_kernel(int M, const float2* gram, float2* coeffs) {
       if (i == j) A[i][j].y = 0.0;
       V[i][j] = make_double2(i == j ? 1.0 : 0.0, 0.0);
     }
+  }
+  __syncwarp();
   for (int sweep = 0; sweep < 32; ++sweep) {
     double off = 0.0, diag = 0.0;
     for (int i = 0; i < M; ++i) {
@@ -945,8 +964,9 @@ __global__ void probe_eigh_kernel(int M, const float2* gram, float2* coeffs) {
         const double t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
         const double c = 1.0 / sqrt(1.0 + t * t);
         const double sn = t * c;
+        __syncwarp();  // every lane has read the pair's entries
         // J = [[c, s], [-s e^{-i phi}, c e^{-i phi}]] on columns (p, q): A <- J^H A J
-        for (int k = 0; k < M; ++k) {  // columns
+        if (k < M) {  // columns
           const double2 akp = A[k][p], akq = A[k][q];
           const double2 aq = make_double2(akq.x * ephr + akq.y * ephi, akq.y * ephr - akq.x * ephi);
           A[k][p] = make_double2(c * akp.x - sn * aq.x, c * akp.y - sn * aq.y);
@@ -956,33 +976,42 @@ __global__ void probe_eigh_kernel(int M, const float2* gram, float2* coeffs) {
           V[k][p] = make_double2(c * vkp.x - sn * vq.x, c * vkp.y - sn * vq.y);
           V[k][q] = make_double2(sn * vkp.x + c * vq.x, sn * vkp.y + c * vq.y);
         }
-        for (int k = 0; k < M; ++k) {  // rows: conjugate of the column transform
+        __syncwarp();
+        if (k < M) {  // rows: conjugate of the column transform
           const double2 apk = A[p][k], aqk = A[q][k];
           const double2 aq = make_double2(aqk.x * ephr - aqk.y * ephi, aqk.y * ephr + aqk.x * ephi);
           A[p][k] = make_double2(c * apk.x - sn * aq.x, c * apk.y - sn * aq.y);
           A[q][k] = make_double2(sn * apk.x + c * aq.x, sn * apk.y + c * aq.y);
         }
-        A[p][q] = make_double2(0.0, 0.0);
-        A[q][p] = make_double2(0.0, 0.0);
-        A[p][p].y = 0.0;
-        A[q][q].y = 0.0;
+        __syncwarp();
+        if (k == 0) {
+          A[p][q] = make_double2(0.0, 0.0);
+          A[q][p] = make_double2(0.0, 0.0);
+          A[p][p].y = 0.0;
+          A[q][q].y = 0.0;
+        }
+        __syncwarp();
       }
     }
   }
-  for (int i = 0; i < M; ++i) {
-    w[i] = A[i][i].x;
-    order[i] = i;
-  }
-  for (int i = 1; i < M; ++i) {  // stable insertion sort, decreasing eigenvalue
-    const int o = order[i];
-    int k = i - 1;
-    while (k >= 0 && w[order[k]] < w[o]) {
-      order[k + 1] = order[k];
-      --k;
+  if (k == 0) {
+    for (int i = 0; i < M; ++i) {
+      w[i] = A[i][i].x;
+      order[i] = i;
     }
-    order[k + 1] = o;
+    for (int i = 1; i < M; ++i) {  // stable insertion sort, decreasing eigenvalue
+      const int o = order[i];
+      int h = i - 1;
+      while (h >= 0 && w[order[h]] < w[o]) {
+        order[h + 1] = order[h];
+        --h;
+      }
+      order[h + 1] = o;
+    }
   }
-  for (int i = 0; i < M; ++i) {
+  __syncwarp();
+  if (k < M) {
+    const int i = k;
     const int col = order[i];
     int big = 0;
     double bmag = -1.0;
