@@ -242,13 +242,25 @@ cudaError_t launch_gemm_bn(int bn, int M, int N, int K, int splits, int kps, LA 
 }
 
 // ------------------------------------------------------------ elementwise
-__global__ void wgrad_reduce_kernel(const float* part, int splits, size_t n, float* dw) {
-  const size_t i = (size_t)blockIdx.x * kEw + threadIdx.x;
-  if (i >= n) return;
+constexpr int kReduceLanes = 32;              // outputs of a block
+constexpr int kReduceGroups = kEw / kReduceLanes;
+
+__global__ void __launch_bounds__(kEw) wgrad_reduce_kernel(const float* __restrict__ part,
+                                                           int splits, size_t n, float* dw) {
+  __shared__ float sums[kReduceGroups][kReduceLanes];
+  const int lane = threadIdx.x % kReduceLanes, group = threadIdx.x / kReduceLanes;
+  const size_t i = (size_t)blockIdx.x * kReduceLanes + lane;
   float s = 0.0f;
-#pragma unroll 16  // (the loads of 16 parts in flight, the sum in order)
-  for (int z = 0; z < splits; ++z) s += part[(size_t)z * n + i];
-  dw[i] = s;
+  if (i < n) {
+#pragma unroll 8  // (the loads of 8 parts in flight, the sum in order)
+    for (int z = group; z < splits; z += kReduceGroups) s += part[(size_t)z * n + i];
+  }
+  sums[group][lane] = s;
+  __syncthreads();
+  if (group == 0 && i < n) {
+    for (int g = 1; g < kReduceGroups; ++g) s += sums[g][lane];
+    dw[i] = s;
+  }
 }
 
 // bias gradient: sum over pixels of dy[:, c]; one block per channel, fixed order
@@ -417,12 +429,12 @@ cudaError_t conv3x3_backward_weight(const bf16* x, const bf16* dy, int nb, int H
                        WgradB{dy, npix, cout}, StoreWgradPartial{wpart, M, cout}, err, s);
   }
   if (e != cudaSuccess) return e;
-  wgrad_reduce_kernel<<<(unsigned)((n + kEw - 1) / kEw), kEw, 0, s>>>(wpart, splits, n, dw);
+  auto blocks = [](size_t v) { return (unsigned)((v + kReduceLanes - 1) / kReduceLanes); };
+  wgrad_reduce_kernel<<<blocks(n), kEw, 0, s>>>(wpart, splits, n, dw);
   if (db) {
     if (bias_parts) {
       bias_partial_kernel<<<kBiasBlocks, kTileThreads, 0, s>>>(dy, npix, cout, part);
-      wgrad_reduce_kernel<<<(unsigned)((cout + kEw - 1) / kEw), kEw, 0, s>>>(part, kBiasBlocks,
-                                                                             cout, db);
+      wgrad_reduce_kernel<<<blocks(cout), kEw, 0, s>>>(part, kBiasBlocks, cout, db);
     } else {
       bias_grad_kernel<<<cout, kEw, 0, s>>>(dy, npix, cout, db);
     }

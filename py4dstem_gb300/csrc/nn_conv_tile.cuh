@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kTileThreads) bias_partial_kernel(const bf16* 
 #pragma unroll
     for (int i = 0; i < 8; ++i) s[i] = 0.0f;
     if (pl < lanes && kc < chunks) {
-#pragma unroll 4
+#pragma unroll 16  // (latency-bound: 16 loads in flight)
       for (int p = p0 + pl; p < p1; p += lanes) {
         const uint4 u = *reinterpret_cast<const uint4*>(dy + (size_t)p * C + 8 * kc);
         const bf16* b = reinterpret_cast<const bf16*>(&u);
