@@ -91,8 +91,8 @@ def parse_args(argv=None):
                     help="learned-init: iterations of the plain run")
     ap.add_argument("--schedule", type=int, default=0,
                     help="128^2 kernel schedule: 0 default (3), 1 shared-memory passes by "
-                         "the whole block, 2 register-resident, 3 shared-memory passes by "
-                         "groups of warps")
+                         "the whole block, 2 register-resident, 3 packed passes by warps "
+                         "that own rows and columns")
     return ap.parse_args(argv)
 
 
@@ -639,7 +639,7 @@ def run_ours(args):
 
     bound_name, _ = _rl.bound(flops_pos, bytes_pos, fp32_peak or 77.0, hbm_peak)
     kernel_name = {1: "position_kernel<128,128,1024,1>", 2: "gd128_kernel"}.get(
-        args.schedule, "wave_gd_kernel<128>")
+        args.schedule, "wave_gd_kernel<128, false>")
     if bound_name == "hbm":
         roof = {"bound": "hbm", "achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": hbm_achieved / hbm_peak, "peak_source": hbm_source + ", of measured"}

@@ -280,27 +280,14 @@ __device__ __forceinline__ float2 cis_rounded(float phi) {
   return make_float2(__fadd_rn(c.hi, c.lo), __fadd_rn(s.hi, s.lo));
 }
 
-// Barriers a pass synchronises its threads with: the whole block, or a named
-// barrier of one group of warps that owns its lines alone (bar.sync id, n;
-// ids 1..15, id 0 being the block barrier).
-struct BlockSync {
-  __device__ __forceinline__ void operator()() const { __syncthreads(); }
-};
-struct GroupSync {
-  int id, threads;
-  __device__ __forceinline__ void operator()() const {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-  }
-};
-
 // One Stockham pass over NLINES lines of length L with radix R; NS is the length
 // of the sub-transforms already completed. Lanes of a warp take consecutive
 // lines, so with a pitch of SY+1 rows (row pass) or unit-stride columns (column
-// pass) the 32 lanes touch 32 distinct banks pairs. The NT threads that own the
-// lines (thread index tid < NT among them) synchronise through `sync`.
-template <int L, int R, int NS, int NLINES, int NT, int DIR, typename Sync>
+// pass) the 32 lanes touch 32 distinct banks pairs. The NT threads of the block
+// share the butterflies.
+template <int L, int R, int NS, int NLINES, int NT, int DIR>
 __device__ __forceinline__ void line_pass(float2* buf, int line_stride, int elem_stride,
-                                          const float2* __restrict__ tw, int tid, Sync sync) {
+                                          const float2* __restrict__ tw, int tid) {
   constexpr int BF = L / R;            // butterflies per line
   constexpr int WORK = NLINES * BF;    // butterflies per pass
   constexpr int ITEMS = (WORK + NT - 1) / NT;
@@ -328,7 +315,7 @@ __device__ __forceinline__ void line_pass(float2* buf, int line_stride, int elem
       dft<R, DIR>(row);
     }
   }
-  sync();
+  __syncthreads();
 #pragma unroll
   for (int it = 0; it < ITEMS; ++it) {
     const int w = tid + it * NT;
@@ -342,15 +329,14 @@ __device__ __forceinline__ void line_pass(float2* buf, int line_stride, int elem
       for (int k = 0; k < R; ++k) p[(base + k * NS) * elem_stride] = v[it][k];
     }
   }
-  sync();
+  __syncthreads();
 }
 
 // Radix schedule per transform length: a compile-time list of passes.
-#define PTY_PASS(L, R, NS) line_pass<L, R, NS, NLINES, NT, DIR>(b, ls, es, tw, tid, sync)
-#define PTY_SCHEDULE_RUN                                                                  \
-  template <int NLINES, int NT, int DIR, typename Sync = BlockSync>                       \
-  __device__ static void run(float2* b, int ls, int es, const float2* tw, int tid,        \
-                             Sync sync = Sync())
+#define PTY_PASS(L, R, NS) line_pass<L, R, NS, NLINES, NT, DIR>(b, ls, es, tw, tid)
+#define PTY_SCHEDULE_RUN                \
+  template <int NLINES, int NT, int DIR> \
+  __device__ static void run(float2* b, int ls, int es, const float2* tw, int tid)
 template <int L>
 struct Schedule;
 template <>

@@ -901,9 +901,15 @@ namespace {
 
 // Square regions run the wave kernels (ptycho_wave.cuh) unless the batch needs
 // the general ones; at 128 x 128 the schedule setting can ask for those too.
+// General -> packed kernel, us: 1024 positions of plain gradient descent at
+// 48 x 48 61 -> 47, 64 x 64 82 -> 59, 96 x 96 247 -> 143, 128 x 128 281 -> 172;
+// 256 positions of 8 slices at 32 x 32 68 -> 55, 64 x 64 195 -> 115; of 4 modes at
+// 64 x 64 133 -> 78. Plain gradient descent at 32 x 32 keeps the general one (24.7,
+// packed 27.2).
 template <int SX, int SY>
 bool use_wave(const BatchArgs& a) {
   const int schedule = get_schedule(SX);
+  if (SX == 32 && wave_plain(a)) return false;
   return SX == SY && (schedule == 0 || schedule == 3) && !small_batch(a) && wave_batch(a);
 }
 

@@ -330,6 +330,10 @@ __device__ __forceinline__ Cx2 tmem_cell(const uint32_t (&r)[32], int k) {
 // kKind 0: plain single-slice single-probe gradient descent; 1: any single-probe
 // model (multislice, projection sets, kept far fields, forward only, exact probe
 // gradient); 2: any mixed-state model (likewise).
+// Bound: shared memory (two round trips an axis) and the L2 traffic of the stashed
+// P_s, patches and terms, one block of 128 x 128 an SM. 256 positions at 128 x 128:
+// 8 slices 490 us (557 with the block-wide walk by groups of warps), 4 modes 324
+// (340); both are 1.7 rounds of 152 blocks and pay two.
 template <int S, int kKind>
 __global__ void __launch_bounds__(WaveFft<S>::NT) wave_position_kernel(BatchArgs a) {
   using W = WaveFft<S>;
@@ -1178,7 +1182,7 @@ cudaError_t launch_wave_position(const BatchArgs& a, cudaStream_t s) {
   void (*fn)(BatchArgs) = wave_mixed(a) ? wave_position_kernel<S, 2> : wave_position_kernel<S, 1>;
   if constexpr (S == 128) {
     if (blocks > 0) fn = wave_plain(a) ? wave_gd_kernel<S, false> : wave_gd_kernel<S, true>;
-  } else {
+  } else if constexpr (S > 32) {
     if (wave_plain(a)) fn = wave_position_kernel<S, 0>;
   }
   cudaError_t e = ensure_smem_limit(reinterpret_cast<const void*>(fn), (int)smem);

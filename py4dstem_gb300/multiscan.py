@@ -188,7 +188,7 @@ class MultiScanReconstruction:
         concs = [True, False] if self.concurrent == "auto" else [bool(self.concurrent)]
         # the 128 x 128 kernel schedule (1: shared-memory transforms by the whole
         # block, 2: register-resident four-step transforms for single-slice
-        # single-probe scans, 3: shared-memory transforms by groups of warps)
+        # single-probe scans, 3: packed transforms by warps that own rows and columns)
         # matters for scans at a 128^2 detector
         eligible = any(tuple(p._region_of_interest_shape) == (128, 128) for p in self.scans)
         scheds = [1, 2, 3] if eligible else [0]
