@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(NT) overlap_accumulate_kernel(BatchArgs a, flo
 // ------------------------------------------------------------------- probe side
 constexpr int kProbeChunkMax = 1024;  // positions per chunk whose patch origins are staged
 
-__global__ void __launch_bounds__(NT) probe_reduce_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(NT, 8) probe_reduce_kernel(BatchArgs a) {
   __shared__ int2 origin[kProbeChunkMax];  // patch origins (pmod'ed) of this chunk's positions
   const int N = a.Sx * a.Sy;
   const int e = blockIdx.x * NT + threadIdx.x;
@@ -418,9 +418,23 @@ __global__ void __launch_bounds__(NT) probe_reduce_kernel(BatchArgs a) {
   const int rlo = c * rper, rhi = min(rows, rlo + rper);
   for (int m = 0; m < a.M; ++m) {
     float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 8
-    for (int b = rlo; b < rhi; ++b) {
-      const float2 v = sp[((size_t)b * a.M + m) * N + e];
+    const size_t stride = (size_t)a.M * N;
+    const float2* p = sp + rlo * stride + (size_t)m * N + e;
+    int b = rlo;
+    // (batches of loads spelled out: left to unrolling, the loads of the two kinds of
+    // rows waited for one another, 33 us instead of 14 for 1024 rows of 32 x 32)
+    for (; b + 8 <= rhi; b += 8, p += 8 * stride) {
+      float2 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = p[i * stride];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        acc.x += v[i].x;
+        acc.y += v[i].y;
+      }
+    }
+    for (; b < rhi; ++b, p += stride) {
+      const float2 v = *p;
       acc.x += v.x;
       acc.y += v.y;
     }
@@ -457,8 +471,16 @@ __global__ void __launch_bounds__(NT) probe_reduce_kernel(BatchArgs a) {
       n += o.x * o.x + o.y * o.y;
     }
   } else {
-#pragma unroll 8
-    for (int b = lo; b < hi; ++b) n += snp[(size_t)b * N + e];
+    const float* p = snp + (size_t)lo * N + e;
+    int b = lo;
+    for (; b + 8 <= hi; b += 8, p += 8 * (size_t)N) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = p[i * (size_t)N];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) n += v[i];
+    }
+    for (; b < hi; ++b, p += N) n += *p;
   }
   a.probe_npart[(size_t)c * N + e] = n;
 }
