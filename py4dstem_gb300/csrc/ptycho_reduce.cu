@@ -94,8 +94,9 @@ constexpr int kRowsPerLane = 8;  // tile rows one lane visits per list entry (ev
 
 // A cluster of C blocks (8 warps each) per 16x16 object tile and slice; warp w of
 // block r takes part 8 r + w of the batch or, for small batches (kInTurn, C = 1),
-// every eighth of the positions that touch the tile, four at a time. Its lanes test 32 positions at a time
-// for a patch that touches the tile (with the tile origin in patch coordinates)
+// every eighth of the positions that touch the tile, four at a time. Its lanes test
+// 32 positions at a time for a patch that touches the tile (with the tile origin in
+// patch coordinates)
 // and the warp then visits the hits in order. For a hit, lane l covers tile column
 // l % 16 of rows l / 16, l / 16 + 2, ..., so each warp load reads two whole
 // 16-sample staged rows (two 128-byte lines of the object term, two 64-byte ones of
