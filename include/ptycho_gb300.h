@@ -513,12 +513,16 @@ int ptycho_gd_batch_noalloc(const ptycho_geometry* geometry, void* object, void*
  * option but projection sets with kept far fields and the position correction
  * of multislice batches, on arrays aligned to 16 bytes; other cases fall back
  * to 1). The default is 3 where it applies, else 1; other square ROIs have only
- * the default. Process-wide; results agree between schedules to float32
- * rounding. Returns the previous setting (0-3), or -PTYCHO_ERR_INVALID_ARGUMENT
+ * the default. Process-wide, and any thread may set it at any time: a call
+ * takes the setting it finds when it begins. Results agree between schedules to
+ * float32 rounding. Returns the previous setting (0-3), or -PTYCHO_ERR_INVALID_ARGUMENT
  * for a schedule outside 0-3 (the setting is then unchanged).
  * No reference counterpart (tuning knob of this library's autotuner).
  */
 int ptycho_set_kernel_schedule(int32_t roi, int32_t schedule);
+
+/* The schedule set for a ROI edge length (0 where none can be set). */
+int ptycho_get_kernel_schedule(int32_t roi);
 
 /*
  * FP32 throughput probe: `blocks` blocks of 256 threads each run `iters`

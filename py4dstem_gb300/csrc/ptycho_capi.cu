@@ -216,6 +216,7 @@ int prepare(const ptycho_geometry* g, int32_t batch, void* workspace, size_t wor
   a.M = g->num_probes;
   a.potential = g->object_is_potential;
   a.B = batch;
+  a.schedule = a.Sx == a.Sy ? get_schedule(a.Sx) : 0;
   bind_workspace(a, workspace, w);
   if (workspace_bytes < w.total_trans) a.trans = nullptr;
   return PTYCHO_OK;
@@ -517,6 +518,8 @@ int ptycho_prepare_stream(void* stream) {
   if (e != cudaSuccess) return cuda_fail(e, "helper stream");
   return PTYCHO_OK;
 }
+
+int ptycho_get_kernel_schedule(int32_t roi) { return get_schedule(roi); }
 
 int ptycho_set_kernel_schedule(int32_t roi, int32_t schedule) {
   if (schedule < 0 || schedule > 3) {

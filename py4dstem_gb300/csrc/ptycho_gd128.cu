@@ -20,6 +20,8 @@
 //
 // Staging outputs are written in y-major order (e' = y * 128 + x), the order in
 // which a warp's lanes hold them (BatchArgs::staging_t = 1).
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 #include "fft_smem.cuh"
@@ -429,22 +431,19 @@ __global__ void __launch_bounds__(NT, 1) gd128_kernel(BatchArgs a) {
 }  // namespace
 
 namespace {
-// 0: default (the shared-memory passes, measured faster on GB300), 1: shared-memory
-// passes, 2: register-resident
-int g_schedule_128 = 0;
+// 0: default (3 where it applies, else 1), 1: block-wide shared-memory passes,
+// 2: register-resident, 3: packed passes by warps that own rows and columns
+std::atomic<int> g_schedule_128{0};
 }
 
 int set_schedule(int roi, int schedule) {
-  if (roi != S) return 0;
-  const int prev = g_schedule_128;
-  g_schedule_128 = schedule;
-  return prev;
+  return roi == S ? g_schedule_128.exchange(schedule) : 0;
 }
 
-int get_schedule(int roi) { return roi == S ? g_schedule_128 : 0; }
+int get_schedule(int roi) { return roi == S ? g_schedule_128.load() : 0; }
 
 bool position_v2_eligible(const BatchArgs& a) {
-  if (g_schedule_128 != 2) return false;
+  if (a.schedule != 2) return false;
   return a.Sx == S && a.Sy == S && a.T == 1 && a.M == 1 && !a.projection && !a.mixed_formula &&
          !a.forward_only && !a.keep_farfield;
 }

@@ -24,6 +24,8 @@ struct BatchArgs {
   float pa, pb, pc;        // projection parameters a, b, c
   int fix_probe;
   int ew_valid;
+  int schedule;            // get_schedule() when the call began: every choice of a kernel and
+                           // of what it stages follows this one reading
   int staging_t;           // staged per-position terms are y-major (e' = y * Sx + x)
   int forward_only;        // forward model and per-position error only, no adjoint
   int keep_farfield;       // single slice: keep FFT2(psi_m) of each position in scratch_f
@@ -146,8 +148,9 @@ cudaError_t launch_object_gaussian(const BatchArgs& a, const double* w, int R, i
 cudaError_t launch_overlap_accumulate(const BatchArgs& a, float* overlap, cudaStream_t s);
 // Register-resident 128 x 128 single-slice GD kernel (ptycho_gd128.cu).
 // set_schedule stores the preferred schedule for a ROI edge (0 default,
-// 1 shared-memory passes, 2 register-resident, 3 shared-memory passes by groups
-// of warps) and returns the previous one; get_schedule reads it.
+// 1 block-wide shared-memory passes, 2 register-resident, 3 packed passes by warps
+// that own rows and columns) and returns the previous one; get_schedule reads it.
+// Any thread may set it at any time: a call reads it once, into BatchArgs::schedule.
 int set_schedule(int roi, int schedule);
 int get_schedule(int roi);
 bool position_v2_eligible(const BatchArgs& a);

@@ -908,9 +908,8 @@ namespace {
 // packed 27.2).
 template <int SX, int SY>
 bool use_wave(const BatchArgs& a) {
-  const int schedule = get_schedule(SX);
   if (SX == 32 && wave_plain(a)) return false;
-  return SX == SY && (schedule == 0 || schedule == 3) && !small_batch(a) && wave_batch(a);
+  return SX == SY && (a.schedule == 0 || a.schedule == 3) && !small_batch(a) && wave_batch(a);
 }
 
 template <int SX, int SY, int NT>
@@ -1001,8 +1000,7 @@ __global__ void __launch_bounds__(NT, 1) probe_intensity_kernel(BatchArgs a) {
 template <int SX, int SY, int NT>
 cudaError_t launch_probe_intensity_t(const BatchArgs& a, cudaStream_t s) {
   if constexpr (SX == SY) {
-    const int schedule = get_schedule(SX);
-    if (schedule == 0 || schedule == 3) return launch_wave_intensity<SX>(a, s);
+    if (a.schedule == 0 || a.schedule == 3) return launch_wave_intensity<SX>(a, s);
   }
   const size_t smem = Layout<SX, SY>::smem_bytes(false);
   {

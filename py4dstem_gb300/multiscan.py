@@ -145,8 +145,7 @@ class MultiScanReconstruction:
     def _graph(self, concurrent: bool):
         # a captured graph holds the kernels chosen at capture time, so it is
         # kept per 128^2 kernel schedule as well
-        key = (concurrent, _native.lib().ptycho_set_kernel_schedule(128, 0))
-        _native.lib().ptycho_set_kernel_schedule(128, key[1])
+        key = (concurrent, _native.lib().ptycho_get_kernel_schedule(128))
         if key not in self._graphs:
             torch = self.torch
             g = torch.cuda.CUDAGraph()

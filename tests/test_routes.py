@@ -1,0 +1,39 @@
+"""Which kernels a call takes, as far as the host decides it: no GPU needed."""
+
+import ctypes
+
+import pytest
+
+from py4dstem_gb300 import _native, multiscan
+
+
+@pytest.fixture(scope="module")
+def lib():
+    return _native.lib()
+
+
+def test_schedule_can_be_read_without_setting_it(lib):
+    prev = lib.ptycho_set_kernel_schedule(128, 2)
+    try:
+        assert lib.ptycho_get_kernel_schedule(128) == 2
+        assert lib.ptycho_get_kernel_schedule(64) == 0
+    finally:
+        lib.ptycho_set_kernel_schedule(128, prev)
+    assert lib.ptycho_get_kernel_schedule(128) == prev
+
+
+def test_multiscan_graph_lookup_leaves_the_schedule_alone(monkeypatch, lib):
+    """Looking up a captured graph must not write the process-wide setting, not
+    even to put it back: other threads' batches read it meanwhile."""
+    calls = []
+
+    class Recorder:
+        def __getattr__(self, name):
+            calls.append(name)
+            return getattr(lib, name)
+
+    monkeypatch.setattr(multiscan._native, "lib", lambda: Recorder())
+    scans = multiscan.MultiScanReconstruction.__new__(multiscan.MultiScanReconstruction)
+    scans._graphs = {(True, lib.ptycho_get_kernel_schedule(128)): "graph"}
+    assert scans._graph(True) == "graph"
+    assert "ptycho_set_kernel_schedule" not in calls
