@@ -487,8 +487,10 @@ int ptycho_kernel_timing(float* total_ms, int32_t* launches);
  * application whose own allocator owns the GPU): same arguments and results
  * without the workspace; the scratch is a fixed 32 MiB array inside the
  * library that each GPU holds from loading the library until exit. Batches
- * needing more scratch than that (ptycho_workspace_bytes) return
- * PTYCHO_ERR_WORKSPACE. The first call on a device looks up the array's
+ * needing more scratch than that return PTYCHO_ERR_WORKSPACE. The least a batch
+ * needs can be below ptycho_workspace_bytes(), which includes room for copies of
+ * large objects; a batch that fits without them runs a kernel that does without
+ * (results equal to float32 rounding). The first call on a device looks up the array's
  * address and should come before any stream capture. All calls share the
  * array: calls that can overlap on the GPU must be serialised on one stream.
  * The batch-chaining flags PTYCHO_FLAG_SPECTRUM_READY, PTYCHO_FLAG_PREPARE_SPECTRUM

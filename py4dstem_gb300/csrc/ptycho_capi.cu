@@ -189,6 +189,13 @@ void bind_workspace(BatchArgs& a, void* base, const Workspace& w) {
 
 namespace {
 
+// layout of a checked geometry
+Workspace layout_of(const ptycho_geometry* g, int32_t batch) {
+  return workspace_layout(g->roi_x, g->roi_y, g->object_x, g->object_y, g->num_slices,
+                          g->num_probes, batch, (g->flags & PTYCHO_FLAG_KEEP_FARFIELD) != 0,
+                          detector_x(g), detector_y(g));
+}
+
 int prepare(const ptycho_geometry* g, int32_t batch, void* workspace, size_t workspace_bytes,
             BatchArgs& a) {
   int st = check_geometry(g);
@@ -197,10 +204,7 @@ int prepare(const ptycho_geometry* g, int32_t batch, void* workspace, size_t wor
   if (!workspace) return fail(PTYCHO_ERR_WORKSPACE, "workspace is null");
   if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
     return fail(PTYCHO_ERR_WORKSPACE, "workspace must be 256-byte aligned");
-  const Workspace w = workspace_layout(g->roi_x, g->roi_y, g->object_x, g->object_y,
-                                       g->num_slices, g->num_probes, batch,
-                                       (g->flags & PTYCHO_FLAG_KEEP_FARFIELD) != 0,
-                                       detector_x(g), detector_y(g));
+  const Workspace w = layout_of(g, batch);
   if (workspace_bytes < w.total)
     return fail(PTYCHO_ERR_WORKSPACE, "workspace of %zu bytes is smaller than the %zu needed",
                 workspace_bytes, w.total);
@@ -257,10 +261,7 @@ int ptycho_geometry_supported(const ptycho_geometry* g) { return check_geometry(
 size_t ptycho_workspace_bytes(const ptycho_geometry* g, int32_t max_batch) {
   if (!g || max_batch < 1) return 0;
   if (check_geometry(g) != PTYCHO_OK) return 0;
-  return workspace_layout(g->roi_x, g->roi_y, g->object_x, g->object_y, g->num_slices,
-                          g->num_probes, max_batch, (g->flags & PTYCHO_FLAG_KEEP_FARFIELD) != 0,
-                          detector_x(g), detector_y(g))
-      .total_trans;
+  return layout_of(g, max_batch).total_trans;
 }
 
 static int run_batch(const ptycho_geometry* g, void* object, void* probe,
@@ -963,7 +964,9 @@ extern "C" int ptycho_gd_batch_noalloc(const ptycho_geometry* g, void* object, v
                 "PTYCHO_FLAG_PREPARE_SPECTRUM or PTYCHO_FLAG_KEEP_FARFIELD (they pass data "
                 "between calls through the scratch, which every call shares)");
   if (batch < 1) return fail(PTYCHO_ERR_INVALID_ARGUMENT, "batch must be >= 1 (got %d)", batch);
-  const size_t need = ptycho_workspace_bytes(g, batch);
+  // (the least workspace: without room for the transmission copies as well the
+  // batch runs the general position kernel)
+  const size_t need = layout_of(g, batch).total;
   if (need > kNoallocScratchBytes)
     return fail(PTYCHO_ERR_WORKSPACE,
                 "batch of %d positions needs %zu bytes of scratch; the fixed no-allocation "

@@ -37,3 +37,17 @@ def test_multiscan_graph_lookup_leaves_the_schedule_alone(monkeypatch, lib):
     scans._graphs = {(True, lib.ptycho_get_kernel_schedule(128)): "graph"}
     assert scans._graph(True) == "graph"
     assert "ptycho_set_kernel_schedule" not in calls
+
+
+@pytest.mark.parametrize("roi,obj,batch", [(32, 1024, 500), (32, 1450, 64), (96, 1000, 60)])
+def test_noalloc_takes_batches_that_fit_without_the_copies(lib, roi, obj, batch):
+    """ptycho_workspace_bytes includes room for copies of the object that a batch can
+    do without: the entry point without allocation refuses by what is needed. (The
+    null object stops the call before any GPU work.)"""
+    g = _native.Geometry(roi, roi, obj, obj, 1, 1, 0, 0)
+    assert lib.ptycho_workspace_bytes(ctypes.byref(g), batch) > 32 << 20
+    p = ctypes.c_void_p(0x1000)
+    assert lib.ptycho_gd_batch_noalloc(ctypes.byref(g), None, p, p, None, p, None, batch, 0.5,
+                                       1.0, 0, None, None, p, None) != 3
+    assert lib.ptycho_gd_batch_noalloc(ctypes.byref(g), None, p, p, None, p, None, 4 * batch + 500,
+                                       0.5, 1.0, 0, None, None, p, None) == 3
