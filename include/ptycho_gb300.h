@@ -557,7 +557,9 @@ int ptycho_fp32_fma_probe(int32_t blocks, int32_t iters, float* sink, void* stre
  * cin) float32 = the gradient wrt x for the gradient dy wrt the convolution's
  * output. backward_weight: dweight (cout, 9, cin) and dbias (cout, or NULL)
  * float32, summed over the batch in a fixed order (workspace:
- * ptycho_nn_conv3x3_wgrad_workspace_bytes).
+ * ptycho_nn_conv3x3_wgrad_workspace_bytes). forward and backward_data need their
+ * bf16 arrays aligned to 16 bytes; backward_weight takes any, and is fastest with
+ * both aligned.
  */
 int ptycho_nn_gemm_bf16(const void* a, const void* b, float* c, int32_t m, int32_t n, int32_t k,
                         int32_t* err_flag, void* stream);

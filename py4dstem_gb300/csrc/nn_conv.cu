@@ -399,14 +399,18 @@ cudaError_t conv3x3_backward_weight(const bf16* x, const bf16* dy, int nb, int H
   const size_t n = (size_t)M * cout;
   const int buffers = wgrad_smem(W + 1, 2) <= 220 * 1024 ? 2 : 1;
   const size_t smem = wgrad_smem(W + 1, buffers);
+  // the tile copies and the bias partials read 16 bytes at a time; x and dy that start
+  // elsewhere take the gathered GEMM and the one-kernel bias sum, which read elements
+  const bool x_aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0;
+  const bool dy_aligned = reinterpret_cast<uintptr_t>(dy) % 16 == 0;
   // bias partials first, then as many weight parts as fit
   const size_t bias_floats = (size_t)kBiasBlocks * cout;
-  const bool bias_parts = part_bytes / sizeof(float) >= bias_floats + n;
+  const bool bias_parts = dy_aligned && part_bytes / sizeof(float) >= bias_floats + n;
   float* wpart = part + (bias_parts ? bias_floats : 0);
   const size_t room = (part_bytes / sizeof(float) - (bias_parts ? bias_floats : 0)) / n;
   int splits;
   cudaError_t e;
-  if (line_fits(nb, H, W) && smem <= 220 * 1024) {
+  if (x_aligned && dy_aligned && line_fits(nb, H, W) && smem <= 220 * 1024) {
     const ConvLine g = conv_line(nb, H, W);
     const int tiles = (g.Q + kWgradPixels - 1) / kWgradPixels;
     const int bm = (cin + kWgradRows - 1) / kWgradRows;
