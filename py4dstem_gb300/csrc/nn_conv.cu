@@ -335,7 +335,7 @@ size_t wgrad_smem(int pitch, int buffers) {
 
 // the padded line of pixels has to fit an int index
 bool line_fits(int nb, int H, int W) {
-  return (size_t)nb * (H + 1) * (W + 1) < (size_t)1 << 30;
+  return (size_t)nb * ((size_t)H + 1) * ((size_t)W + 1) < (size_t)1 << 30;
 }
 
 cudaError_t conv3x3_forward(const bf16* x, int nb, int H, int W, int cin, const bf16* w,
@@ -380,6 +380,8 @@ size_t conv3x3_wgrad_workspace_min(int nb, int H, int W, int cin, int cout) {
 }
 
 size_t conv3x3_wgrad_workspace(int nb, int H, int W, int cin, int cout) {
+  const size_t least = conv3x3_wgrad_workspace_min(nb, H, W, cin, cout);
+  if (!line_fits(nb, H, W)) return least;  // (the gathered GEMM's parts)
   const int tiles = (nb * (H + 1) * (W + 1) + kWgradPixels - 1) / kWgradPixels;
   const int blocks = ((cin + kWgradRows - 1) / kWgradRows) *
                      ((cout + kWgradColumns - 1) / kWgradColumns);
@@ -387,7 +389,6 @@ size_t conv3x3_wgrad_workspace(int nb, int H, int W, int cin, int cout) {
   if (splits > tiles) splits = tiles;
   const size_t want = sizeof(float) * ((size_t)splits * 9 * cin * cout +
                                        (size_t)kBiasBlocks * cout);
-  const size_t least = conv3x3_wgrad_workspace_min(nb, H, W, cin, cout);
   return want > least ? want : least;
 }
 

@@ -51,3 +51,11 @@ def test_noalloc_takes_batches_that_fit_without_the_copies(lib, roi, obj, batch)
                                        1.0, 0, None, None, p, None) != 3
     assert lib.ptycho_gd_batch_noalloc(ctypes.byref(g), None, p, p, None, p, None, 4 * batch + 500,
                                        0.5, 1.0, 0, None, None, p, None) == 3
+
+
+@pytest.mark.parametrize("nb,H,W", [(1, 1, 1 << 30), (1, 1 << 20, 1 << 10), (255, 2895, 2896)])
+def test_wgrad_workspace_of_the_largest_images(lib, nb, H, W):
+    """Near 2^31 pixels the padded line of pixels no longer fits an int: the parts
+    of the gathered GEMM, at most 64, are all the workspace that is asked for."""
+    parts = 4 * 9 * 16 * 32
+    assert lib.ptycho_nn_conv3x3_wgrad_workspace_bytes(nb, H, W, 16, 32) == 64 * parts
