@@ -188,13 +188,16 @@ __global__ void __launch_bounds__(NT, kInTurn ? 1 : 4) object_reduce_kernel(Batc
   for (int base = b0; base < b1; base += 32) {
     const int i = base + lane;
     bool hit = false;
-    int d = 0;  // (dx << 16) | dy
+    // (dx << 16) | dy of a hit, each counted from -(tile edge - 1) where the tile
+    // starts before the patch, so that both fit 16 bits on objects of any size
+    int d = 0;
     if (i < b1) {
       const int2 r = a.pos_round[i];
       const int dx = pmod(tx0 - (r.x + fminx), a.Px);
       const int dy = pmod(ty0 - (r.y + fminy), a.Py);
-      hit = (dx < a.Sx || dx + tw - 1 >= a.Px) && (dy < a.Sy || dy + th - 1 >= a.Py);
-      d = (dx << 16) | dy;
+      const bool wx = dx + tw - 1 >= a.Px, wy = dy + th - 1 >= a.Py;
+      hit = (dx < a.Sx || wx) && (dy < a.Sy || wy);
+      d = (int)((unsigned)(wx ? dx - a.Px : dx) << 16) | ((wy ? dy - a.Py : dy) & 0xffff);
     }
     unsigned hits = __ballot_sync(0xffffffffu, hit);
     if (kInTurn) {
@@ -213,11 +216,12 @@ __global__ void __launch_bounds__(NT, kInTurn ? 1 : 4) object_reduce_kernel(Batc
       const int bit = __ffs(hits) - 1;
       hits &= hits - 1;
       const int du0 = __shfl_sync(0xffffffffu, d, bit);
-      const int du = tr ? (du0 & 0xffff) : (du0 >> 16);
-      const int dv = tr ? (du0 >> 16) : (du0 & 0xffff);
+      const int dx = du0 >> 16, dy = (int)((unsigned)du0 << 16) >> 16;
+      const int du = tr ? dy : dx;
+      const int dv = tr ? dx : dy;
       // this lane's column: patch coordinate sv (one object wrap at most)
       int sv = dv + iv;
-      if (sv >= Pv) sv -= Pv;
+      if (sv < 0) sv += Pv;
       const bool vok = iv < tv && sv < Sv;
       const int lv = sv >= hv ? sv - hv : sv + hv;
       const size_t col = (size_t)(base + bit) * N + lv;
@@ -225,7 +229,7 @@ __global__ void __launch_bounds__(NT, kInTurn ? 1 : 4) object_reduce_kernel(Batc
       for (int k = 0; k < kRowsPerLane; ++k) {
         const int iu = iu0 + 2 * k;
         int su = du + iu;
-        if (su >= Pu) su -= Pu;
+        if (su < 0) su += Pu;
         v[h][k] = make_float2(0.f, 0.f);
         w[h][k] = 0.f;
         if (vok && iu < tu && su < Su) {
