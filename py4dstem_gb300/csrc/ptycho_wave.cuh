@@ -36,9 +36,11 @@ __host__ __device__ __forceinline__ int transmission_pitch(int Py, int S) {
 }
 
 __global__ void __launch_bounds__(256) transmission_kernel(BatchArgs a, int pitch) {
-  const int c = blockIdx.x * 256 + threadIdx.x;  // cell of the row
+  // (rows and the parts of a row in one grid axis: the others end at 65535)
+  const int parts = (pitch + 255) / 256;
+  const int x = blockIdx.x / parts, s = blockIdx.y;
+  const int c = blockIdx.x % parts * 256 + threadIdx.x;  // cell of the row
   if (c >= pitch) return;
-  const int x = blockIdx.y, s = blockIdx.z;
   const size_t row = ((size_t)s * a.Px + x) * a.Py;
   float2 v[3];
 #pragma unroll
@@ -61,7 +63,7 @@ __global__ void __launch_bounds__(256) transmission_kernel(BatchArgs a, int pitc
 
 inline cudaError_t launch_transmission(const BatchArgs& a, cudaStream_t s) {
   const int pitch = transmission_pitch(a.Py, a.Sy);
-  transmission_kernel<<<dim3((pitch + 255) / 256, a.Px, a.T), 256, 0, s>>>(a, pitch);
+  transmission_kernel<<<dim3((pitch + 255) / 256 * a.Px, a.T), 256, 0, s>>>(a, pitch);
   return cudaGetLastError();
 }
 

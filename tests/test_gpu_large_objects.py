@@ -38,3 +38,9 @@ def test_tiles_of_long_objects(cuda, length, axis):
     pos = [(40.0 + 3 * i, x + (length - 40000 if i > 3 else 0)) for i, x in enumerate(LONG)]
     shape = (80, length) if axis else (length, 80)
     _check(48, shape, pos if axis else [p[::-1] for p in pos])
+
+
+def test_copies_of_long_objects(cuda):
+    """More rows than a grid's second axis holds (65535), on a packed kernel."""
+    _check(96, (70000, 128), [(x + (30000 if i > 3 else 0), 60.0 + 3 * i)
+                              for i, x in enumerate(LONG)])
