@@ -941,7 +941,11 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
   float* const gx = a.st_nobj + (size_t)b * N;
   float* const gy = a.st_nprobe + (size_t)b * N;
   const float* amp = a.amplitudes + (size_t)arow * N;
+  // sums of the normal equations: float over the 16 samples of a task, as many as a
+  // thread of the block-wide walk adds at 128 x 128
   float sxx = 0.f, sxy = 0.f, syy = 0.f, sxd = 0.f, syd = 0.f;
+  float first[5] = {0.f, 0.f, 0.f, 0.f, 0.f};  // task 0's where a thread has two
+  static_assert(W::TITER <= 2, "tasks of a thread");
 #pragma unroll 1
   for (int m = 0; m < M; ++m) {
     const float2* __restrict__ spec = a.probe_spec + (size_t)m * N;
@@ -1011,6 +1015,14 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
         if (W::TASKS % 32 != 0 && t >= W::TASKS) break;
         Cx2 r[8], v[8];
         const uint32_t tf = tm + 32 * (W::TITER + it);
+        if (W::TITER > 1 && last && it == 1) {
+          first[0] = sxx;
+          first[1] = sxy;
+          first[2] = syy;
+          first[3] = sxd;
+          first[4] = syd;
+          sxx = sxy = syy = sxd = syd = 0.f;
+        }
         if (!kTmem || dir == 0) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) r[i] = from_pair(ld_cell(f0 + p.fourier(t, i)));
@@ -1062,22 +1074,31 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchAr
       __syncthreads();  // the wave is rewritten by rows (dir 1) or the next mode
     }
   }
-  // the block's sums, in double: a warp per sum over the threads' partials (the
-  // wave's shared memory is free by now)
+  // the block's sums over the tasks' partials (the wave's shared memory is free by
+  // now): a warp per sum, each lane adding its partials as a float and the sum of the
+  // rounding errors (TwoSum, so about 46 bits), the lanes in double. (Partials added in
+  // double cost 2.5 us a position with two tasks a thread: conversions and additions
+  // run at a sixtieth of the float rate.)
   float* const part = reinterpret_cast<float*>(smem4);
-  part[tid] = sxx;
-  part[W::NT + tid] = sxy;
-  part[2 * W::NT + tid] = syy;
-  part[3 * W::NT + tid] = sxd;
-  part[4 * W::NT + tid] = syd;
+  const float last_task[5] = {sxx, sxy, syy, sxd, syd};
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    part[k * W::NT + tid] = last_task[k];
+    if (W::TITER > 1) part[(5 + k) * W::NT + tid] = first[k];
+  }
   __syncthreads();
   for (int k = w.warp; k < 5; k += W::WARPS) {
-    double x = 0.0;
+    cis_detail::DF x{part[k * W::NT + w.lane], 0.0f};
 #pragma unroll
-    for (int j = 0; j < W::WARPS; ++j) x += part[k * W::NT + 32 * j + w.lane];
+    for (int j = 1; j < W::TITER * W::WARPS; ++j) {
+      const cis_detail::DF t = cis_detail::two_sum(
+          x.hi, part[(j / W::WARPS * 5 + k) * W::NT + 32 * (j % W::WARPS) + w.lane]);
+      x = {t.hi, __fadd_rn(x.lo, t.lo)};
+    }
+    double sum = (double)x.hi + x.lo;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (w.lane == 0) sums[k] = x;
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (w.lane == 0) sums[k] = sum;
   }
   __syncthreads();
   if (tid == 0) correction_update(a, prow, posx, posy, pos_ok, sums);
