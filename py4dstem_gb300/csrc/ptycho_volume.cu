@@ -223,14 +223,23 @@ __global__ void volume_affine_kernel(const double* __restrict__ c, void* out, in
 // ---------------------------------------------------- float32 results: float pairs
 // The same rotation for float32 results (out_mode 0 and 2) on the float32 units:
 // every coefficient, weight, coordinate and sum is an unevaluated pair hi + lo of
-// floats (about 46 bits), rounded once at the end, so the results are the floats
-// that float64 arithmetic gives but where a sum falls within 1e-6 ulp of a tie.
+// floats (about 46 bits), rounded once at the end. These are fewer bits than the 53
+// of float64, in float64 input too: a result is within half an ulp and 1e-12 of the
+// largest coefficient of the exact one (a coordinate near 100 carries an error of
+// about 1e-12), so where a value is small against its neighbours' coefficients it can
+// be another float than float64 arithmetic gives. Over a 96 x 160 x 160 volume the
+// error against 64 bits is that of the final rounding (6.5e-8) either way.
+// The sums and products are the error-free transformations TwoSum (Knuth) and
+// TwoProduct with a fused multiply-add (Ogita, Rump and Oishi 2005).
 // GB300 does 60 times as many float32 as float64 operations: 96 x 160 x 160 voxels
 // took 1286 us of resampling and 3 x 98 us of prefilters in float64.
 //
-// The coefficients carry a factor 2^-8, which keeps the gain of the filters
-// (6 per axis) inside float range for every finite float volume.
-constexpr float kPairScale = 256.0f;
+// The coefficients carry a factor 2^-9. With the gain of the filters (6 per axis,
+// 216 in all, applied first) the causal recursion reaches 216 / (1 - |pole|) = 295
+// times the largest voxel and the anticausal one adds at most 108 to that: 403, so
+// every finite float volume stays in range. Below about 1e-28 the error terms of the
+// pairs run out of exponents: there the error is up to 2^-135.
+constexpr float kPairScale = 512.0f;
 
 __device__ __forceinline__ float2 pair_of(double v) {
   const float hi = (float)v;
@@ -327,10 +336,10 @@ __global__ void __launch_bounds__(32) pair_prefilter_kernel(const void* __restri
   const bool active = line < lines;
   const int nl = (int)(lines - first < 32 ? lines - first : 32);
   auto load = [&](size_t at) {
-    const double v = in_is_double ? static_cast<const double*>(in)[at] : 0.0;
-    const float2 x = in_is_double ? pair_of(v)
-                                  : make_float2(static_cast<const float*>(in)[at], 0.0f);
-    return pair_mul(x, make_float2(gain, 0.0f));
+    return in_is_double
+               ? pair_of(static_cast<const double*>(in)[at] * (double)gain)
+               : pair_mul(make_float2(static_cast<const float*>(in)[at], 0.0f),
+                          make_float2(gain, 0.0f));
   };
   size_t base = 0, stride = 1;
   if (axis == 2) {
@@ -469,9 +478,11 @@ __global__ void __launch_bounds__(kThreads) pair_affine_kernel(const float2* __r
       float* dst = out + out_row + oh * stride[ax.h];
       if (out_mode == 0) {
         *dst = __fadd_rn(hi, lo);
-      } else {
+      } else if (fabsf(hi) < 1e38f && fabsf(*dst) < 1e38f) {
         const float2 sum = pair_sum(*dst, hi);
         *dst = __fadd_rn(sum.x, __fadd_rn(sum.y, lo));
+      } else {  // (TwoSum is not for sums beyond the float range)
+        *dst = (float)((double)*dst + (double)kPairScale * ((double)value.x + (double)value.y));
       }
     }
   }
