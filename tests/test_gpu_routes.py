@@ -95,3 +95,55 @@ def test_noalloc_and_least_workspace(cuda, S, obj, J):
                 np.testing.assert_array_equal(a, b)
             else:
                 assert rel(a, b) < 2e-6
+
+
+def _iteration(torch, st, offset, projection=False, correction=False, graph=False):
+    J, S = st.amplitudes.shape[0], st.amplitudes.shape[-1]
+    flat = torch.zeros(J * S * S + 4, dtype=torch.float32, device="cuda")
+    amps = flat[offset:offset + J * S * S].reshape(J, S, S)
+    amps.copy_(torch.from_numpy(st.amplitudes))
+    s = engine.create_state(
+        roi_shape=(S, S), object_array=st.object, probe_array=st.probe, amplitudes=amps,
+        positions_px=st.positions_px, num_slices=st.num_slices, num_probes=st.num_probes,
+        potential=False, max_batch=J - 1, propagators=st.propagators, projection=projection,
+        mixed_state=st.mixed, positions_initial=st.positions_px if correction else None)
+    assert s.amplitudes.data_ptr() % 16 == 4 * offset
+    drv = engine.IterationDriver(
+        s, max_batch=J - 1, projection=projection, step_size=0.5, graph=graph,
+        projection_abc=(-1.0, 1.0, 2.0) if projection else (0.0, 0.0, 0.0),
+        mean_intensity=st.mean_intensity, fix_probe_com=False, orthogonalize_probe=False,
+        **(dict(position_correction=dict(step_size=0.9, max_update_px=0.5, max_total_px=2.0,
+                                         center_of_mass=False)) if correction else {}))
+    order = np.arange(J) if projection else np.random.default_rng(1).permutation(J)
+    drv.iterate(order)
+    if graph:
+        for _ in range(2):
+            drv.iterate(order)
+    torch.cuda.synchronize()
+    return [t.cpu().numpy() for t in (s.object, s.probe, s.error_accum, s.positions)]
+
+
+@pytest.mark.parametrize("model", [dict(), dict(slices=2), dict(modes=2), dict(slices=2, modes=2)])
+@pytest.mark.parametrize("kind", ["gd", "projection", "correction"])
+@pytest.mark.parametrize("offset", [1, 2])
+def test_amplitudes_off_a_boundary(cuda, model, kind, offset):
+    """128 x 128 amplitudes that start 4 or 8 bytes off a 16-byte boundary go through
+    an aligned copy to the same kernels: the same bits. (Multislice correction and
+    batches that keep the far field of projection sets have one kernel anyway.)"""
+    st = make_state(S=128, J=11, seed=29, **model)
+    kw = dict(projection=kind == "projection", correction=kind == "correction")
+    want = _iteration(cuda, st, 0, **kw)
+    got = _iteration(cuda, st, offset, **kw)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_amplitudes_off_a_boundary_in_a_graph(cuda):
+    """The same inside a captured iteration, and a 96 x 96 batch (general kernel,
+    float32 rounding)."""
+    st = make_state(S=128, J=11, seed=30)
+    for a, b in zip(_iteration(cuda, st, 3, graph=True), _iteration(cuda, st, 0, graph=True)):
+        np.testing.assert_array_equal(a, b)
+    st = make_state(S=96, J=11, seed=31)
+    for a, b in zip(_iteration(cuda, st, 1), _iteration(cuda, st, 0)):
+        assert rel(a, b) < 2e-6
