@@ -147,3 +147,40 @@ def test_amplitudes_off_a_boundary_in_a_graph(cuda):
     st = make_state(S=96, J=11, seed=31)
     for a, b in zip(_iteration(cuda, st, 1), _iteration(cuda, st, 0)):
         assert rel(a, b) < 2e-6
+
+
+@pytest.mark.parametrize("S", [32, 48, 64])
+def test_correction_of_small_and_large_batches(cuda, S):
+    """A position's correction does not depend on how many others share its batch:
+    40 positions corrected alone and among 300, with nothing else updated, move by
+    the same bits. (Positions near 0, where float32 shows the last bits of a move.)"""
+    torch = cuda
+    lib = _native.lib()
+    J, few = 300, 40
+    st = make_state(S=S, J=J, seed=S, obj_px=S + 24)
+    pos = np.random.default_rng(S).uniform(-0.4, 0.4, size=(J, 2)).astype(np.float32)
+
+    def moved(n):
+        s = engine.create_state(
+            roi_shape=(S, S), object_array=st.object, probe_array=st.probe,
+            amplitudes=st.amplitudes, positions_px=pos, num_slices=1, num_probes=1,
+            potential=False, max_batch=J, positions_initial=pos)
+        s.geometry.flags |= _native.FLAG_KEEP_FARFIELD
+        nbytes = int(lib.ptycho_workspace_bytes(ctypes.byref(s.geometry), J))
+        ws = torch.empty(nbytes + 256, dtype=torch.uint8, device="cuda")
+        ws_ptr = ctypes.c_void_p((ws.data_ptr() + 255) & ~255)
+        assert lib.ptycho_gd_batch(
+            ctypes.byref(s.geometry), engine._ptr(s.object), engine._ptr(s.probe),
+            engine._ptr(s.amplitudes), None, engine._ptr(s.positions), None, n, 0.0, 1.0, 1,
+            None, None, engine._ptr(s.error_accum), ws_ptr, nbytes, engine._stream()) == 0
+        assert lib.ptycho_position_correction(
+            ctypes.byref(s.geometry), engine._ptr(s.object), engine._ptr(s.probe), None,
+            engine._ptr(s.amplitudes), None, engine._ptr(s.positions),
+            engine._ptr(s.positions_initial), None, n, 0.9, 0.5, 2.0, ws_ptr, nbytes,
+            engine._stream()) == 0
+        torch.cuda.synchronize()
+        return s.positions.cpu().numpy()
+
+    a, b = moved(few), moved(J)
+    assert np.all(a[few:] == pos[few:]) and np.all(np.any(a[:few] != pos[:few], axis=1))
+    np.testing.assert_array_equal(a[:few], b[:few])
