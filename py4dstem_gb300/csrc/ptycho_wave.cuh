@@ -218,9 +218,13 @@ __device__ __noinline__ float3 project_lane(bool gd, float A, float re, float im
 
 // The Fourier projection of a task's eight cells: |f| and A / |f| from one
 // reciprocal square root and Newton steps on the residuals s - |f|^2 and
-// A - q |f|, packed (both within an ulp of the IEEE square root and quotient,
-// where those took 25 instructions a sample). A task with a square outside
-// [1e-30, 1e30] other than 0 takes project_lane.
+// A - q |f|, packed, where the IEEE square root and quotient took 25 instructions a
+// sample. Each residual is one fused multiply-add, so a step ends in one rounding of a
+// value accurate to about 2^-45 (the method: P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990): the results are the
+// correctly rounded ones but for values that close to a tie. Restated with any error
+// the reciprocal root may have, one in 2e6 differs, by an ulp; here none of 2e8 did. A
+// task with a square outside [1e-30, 1e30] other than 0 takes project_lane.
 __device__ __forceinline__ void project(bool gd, const float2 (&A)[8], Cx2 (&f)[8], float2& err) {
   float2 s[8], g[8];  // |f|^2, and the same with 1 for 0
   float lo = 1.0f, hi = 1.0f;
