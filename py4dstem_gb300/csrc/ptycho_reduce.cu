@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(NT, kInTurn ? 1 : 4) object_reduce_kernel(Batc
       const int bit = __ffs(hits) - 1;
       hits &= hits - 1;
       const int du0 = __shfl_sync(0xffffffffu, d, bit);
-      const int dx = du0 >> 16, dy = (int)((unsigned)du0 << 16) >> 16;
+      const int dx = du0 >> 16, dy = (int16_t)du0;
       const int du = tr ? dy : dx;
       const int dv = tr ? dx : dy;
       // this lane's column: patch coordinate sv (one object wrap at most)

@@ -36,10 +36,9 @@ __host__ __device__ __forceinline__ int transmission_pitch(int Py, int S) {
 }
 
 __global__ void __launch_bounds__(256) transmission_kernel(BatchArgs a, int pitch) {
-  // (rows and the parts of a row in one grid axis: the others end at 65535)
-  const int parts = (pitch + 255) / 256;
-  const int x = blockIdx.x / parts, s = blockIdx.y;
-  const int c = blockIdx.x % parts * 256 + threadIdx.x;  // cell of the row
+  // (rows on the first grid axis: the others end at 65535)
+  const int x = blockIdx.x, s = blockIdx.z;
+  const int c = blockIdx.y * 256 + threadIdx.x;  // cell of the row
   if (c >= pitch) return;
   const size_t row = ((size_t)s * a.Px + x) * a.Py;
   float2 v[3];
@@ -63,7 +62,7 @@ __global__ void __launch_bounds__(256) transmission_kernel(BatchArgs a, int pitc
 
 inline cudaError_t launch_transmission(const BatchArgs& a, cudaStream_t s) {
   const int pitch = transmission_pitch(a.Py, a.Sy);
-  transmission_kernel<<<dim3((pitch + 255) / 256 * a.Px, a.T), 256, 0, s>>>(a, pitch);
+  transmission_kernel<<<dim3(a.Px, (pitch + 255) / 256, a.T), 256, 0, s>>>(a, pitch);
   return cudaGetLastError();
 }
 
@@ -669,8 +668,9 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_position_kernel(BatchArgs
 // 128 KB out and back through L2), and the probe terms conj(O) chi of the
 // block's positions are summed there too and leave once per block, as row
 // blockIdx.x of st_probe (probe_reduce_kernel then adds gridDim.x rows instead
-// of B). Positions go to blocks by index, so every sum has a fixed order. The
-// next position's amplitudes and ramps are fetched while this one's adjoint runs.
+// of B). Positions go to blocks by index, so every sum has a fixed order. A
+// position's amplitudes travel while its first column and row passes run; the spectrum
+// and ramps of the next position follow this one's adjoint.
 // 128 x 128, per 1024 positions: 172 us, where the block-wide walk with named
 // barriers took 250 and one position per block of this one 219.
 // kFull adds the projection sets and the kept far field: 4096 positions of a
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(WaveFft<S>::NT) wave_gd_kernel(BatchArgs a) {
 // direction. For a single probe at 128 x 128 (kTmem) the blocks are resident and
 // the probe and the far field of the batch wait in tensor memory, the x derivative
 // in shared memory. Bound: L2 traffic, 580 KB a position (1090 through memory).
-// 128 x 128, 1024 positions: 197 us; through memory, with the sums of all threads
+// 128 x 128, 1024 positions: 191 us; through memory, with the sums of all threads
 // in double: 303; the block-wide walk: 465.
 template <int S, bool kTmem>
 __global__ void __launch_bounds__(WaveFft<S>::NT) wave_correction_kernel(BatchArgs a) {
@@ -1196,7 +1196,8 @@ cudaError_t realign_amplitudes(BatchArgs& a, float* room, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// They also need room for the transmission copies in the workspace (a.trans).
+// They also need room for the transmission copies in the workspace (a.trans;
+// ptycho_workspace_bytes() includes it, a caller's workspace may hold less).
 // Projection sets that keep the far field of psi (position correction) run the
 // general kernel.
 inline bool wave_batch(const BatchArgs& a) {
