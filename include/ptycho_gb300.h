@@ -513,8 +513,8 @@ int ptycho_gd_batch_noalloc(const ptycho_geometry* geometry, void* object, void*
  * shared-memory passes by warps that each own 8 rows / columns, with block-wide
  * barriers only between the axes of a transform (128 x 128: every model and
  * option but projection sets with kept far fields and the position correction
- * of multislice batches, on arrays aligned to 16 bytes; other cases fall back
- * to 1). The default is 3 where it applies, else 1; other square ROIs have only
+ * of multislice batches, on amplitudes of any alignment and other arrays aligned
+ * to 16 bytes (the mask to 8); other cases fall back to 1). The default is 3 where it applies, else 1; other square ROIs have only
  * the default. Process-wide, and any thread may set it at any time: a call
  * takes the setting it finds when it begins. Results agree between schedules to
  * float32 rounding. Returns the previous setting (0-3), or -PTYCHO_ERR_INVALID_ARGUMENT

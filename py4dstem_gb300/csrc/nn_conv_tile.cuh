@@ -20,6 +20,10 @@
 //                             K = pixels (both operands MN-major, same layout); one
 //                             accumulator per tap
 //
+// The zeros take part in the products, on both sides of the weight gradient: an
+// infinite or NaN activation at an image's border reaches the taps that pair it
+// with the zeros too (0 x inf), beside those that pair it with gradients.
+//
 // Bound: the copy of the tiles from L2 (about twice the input) and, for narrow
 // layers, the A operand's 4 KB per MMA. Every wait is bounded as in tc_gemm.cuh.
 #pragma once

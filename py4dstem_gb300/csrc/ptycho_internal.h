@@ -106,11 +106,15 @@ bool roi_supported(int Sx, int Sy);
 // (reported by ptycho_read_error as PTYCHO_ERR_NONFINITE).
 __device__ __forceinline__ float finite_or_zero(float v) { return isfinite(v) ? v : 0.0f; }
 
-// Small batches of single-probe gradient descent on detectors up to 64 x 64 run the
-// general position kernel with twice its threads, as fast there as the packed one
-// (64 x 64, batch 64: both 14.7 us), and sum each object pixel over its positions in
-// turn: the error series of a reconstruction, which is reported in float64, keeps
-// its last bit that way.
+// Batches of at most 256 positions of plain gradient descent on detectors up to
+// 64 x 64 keep the arithmetic and the order of sums of the general position kernel, a
+// rule of compatibility: the error series of a reconstruction is reported in float64
+// and compared by its bits, and small scans run such batches (a larger batch's series
+// is equal to float32 rounding). They run that kernel with twice its threads. A whole
+// batch, us, so / with the packed kernel: 32 x 32, 64 positions 19.9 / 24.2, 256
+// 28.7 / 31.1; 48 x 48, 64 26.2 / 28.9, 256 44.4 / 39.1; 64 x 64, 64 29.8 / 29.1, 128
+// 33.2 / 31.3, 256 52.6 / 42.7: it costs nothing up to one position an SM and up to a
+// fifth at two rounds of them.
 inline bool small_batch(const BatchArgs& a) {
   return a.B <= 256 && a.Sx * a.Sy <= 64 * 64 && a.T == 1 && a.M == 1 && !a.mixed_formula &&
          !a.projection && !a.forward_only && !a.keep_farfield && !a.exact_probe_grad;

@@ -915,7 +915,7 @@ bool use_wave(const BatchArgs& a) {
 // The correction of a single-slice batch has no such exceptions (and its arguments
 // say nothing of the batch it follows). General -> packed kernel, us: 32 x 32, 64
 // positions 16.3 -> 11.7, 1024 40.4 -> 25.9; 48 x 48, 64 26.2 -> 13.6, 256 50.0 -> 16.5;
-// 64 x 64, 64 28.9 -> 14.9, 256 56.6 -> 19.8; 128 x 128, 1024 465 -> 196.
+// 64 x 64, 64 28.9 -> 14.9, 256 56.6 -> 19.8; 128 x 128, 1024 465 -> 191.
 template <int SX, int SY>
 bool use_wave_correction(const BatchArgs& a) {
   return SX == SY && a.T == 1 && (a.schedule == 0 || a.schedule == 3) && wave_batch(a);
