@@ -228,8 +228,8 @@ __global__ void volume_affine_kernel(const double* __restrict__ c, void* out, in
 // largest coefficient of the exact one (a coordinate near 100 carries an error of
 // about 1e-12), so where a value is small against its neighbours' coefficients it can
 // be another float than float64 arithmetic gives. Over 25 volumes of 24 x 40 x 40 to
-// 96 x 160 x 160 voxels, 221 of 2.1e7 results are, each by an ulp, and the error
-// against 64 bits is that of the final rounding either way (their ratio 1.000000).
+// 96 x 160 x 160 voxels, 221 of 2.1e7 results are, by at most 9e-9 of the largest value, and the
+// error against 64 bits is that of the final rounding either way (ratio 1.000000).
 // The sums and products are the error-free transformations TwoSum (Knuth) and
 // TwoProduct with a fused multiply-add (Ogita, Rump and Oishi 2005).
 // GB300 does 60 times as many float32 as float64 operations: 96 x 160 x 160 voxels
